@@ -10,7 +10,11 @@
 // concatenation [sinks, topk] to a multiple of 128, which drops an implementation-defined subset;
 // here the dropped entries are the lowest-ranked ones and the output is sorted.
 //
-// Algorithm per row (1024 threads):
+// Three kernels, chosen by launch_topk_select: the streaming kernel (one sweep over the row, candidates above a sampled
+// bound), and for budgets whose candidates do not fit in shared memory the register-resident kernel (rows of up to
+// 32,768 keys) or the general one described here (any row).
+//
+// Algorithm of the general kernel, per row (1024 threads):
 //   1. map scores to order-preserving 32-bit keys (NaN highest; sinks get key 0, below every real
 //      key) and stage the row in shared memory when it fits (<= ~200 KB), else re-read it from L2;
 //   2. MSB-first radix select, four 8-bit passes with warp-aggregated shared-memory histograms,
@@ -18,7 +22,6 @@
 //   3. one counting sweep and one writing sweep compact the selected indices in index order with
 //      warp ballots: element j is taken if it is a sink, or key > T, or key == T and fewer than
 //      `need` equal keys precede it.
-// The kernel is bandwidth-bound: each score is read once from HBM.
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -471,13 +474,351 @@ __global__ void __launch_bounds__(kRT, 1) topk_select_reg_kernel(const TopkParam
   cp_async_wait_all();
 }
 
+
+// ------------------------------------------------------------------------------------------
+// Streaming kernel: the row is read once, and only candidates are kept.
+//
+// What bounds the selection is instructions per key, not bytes: a key that goes through a histogram pass costs some
+// fifteen of them, and the kernels above take every key through several.  Here a sample of the row (one key in L / 4096)
+// gives a lower bound t below the k-th largest key; one sweep over the row then costs a compare and a conditional add
+// per key and keeps the (key, index) pairs above t - about 1.4 k of them at k = 4096, L = 98,280.  The exact k-th key is
+// found among those by three histogram passes of 11, 11 and 10 bits, and the ascending output comes from a bitmap of the
+// row: one bit per selected index, a scan over the words' population counts, and a staging buffer, so that the order in
+// which warps append candidates does not matter.  A row on which the sample misjudges (fewer than k keys above t and
+// not the tie group at t itself, or more candidates than fit) is selected by the same passes over global memory: the
+// sample decides the time only, never the result.
+// Measured (one B200): 3,840 rows of 98,280 keys, k = 4,096: 8,070 -> 670 us (1.57 GB, floor 240 us at the measured copy
+// rate); the top-p update step of 8 heads x 16,380 keys, which spent 386 us here: 2,194 -> 1,884 us in all.
+// ------------------------------------------------------------------------------------------
+constexpr int kST = 512;                  // threads of the streaming kernel
+constexpr int kSW = kST / 32;
+constexpr int kSU = 4;                    // 16-byte loads of a thread in flight (and as many being processed)
+constexpr int kSample = 4096;
+constexpr int kSampleAll = 8192;          // rows of up to this length: every key is a candidate, no sample
+constexpr int kDigits = 2048;
+constexpr int kStreamMaxL = 131072;       // word prefixes are kept as 16-bit numbers in the histogram's space
+
+struct SharedStream {
+  uint32_t hist[kDigits];
+  uint32_t warp_tot[kSW];
+  uint32_t digit, rem, n_eq;              // result of the last histogram search
+  uint32_t n_cand, n_dead, n_tie;
+};
+
+// rank in the sample that lies below rank k of the row by 4.5 standard deviations of the sampling noise
+__host__ __device__ inline int sample_rank(int k, int L) {
+  const float e = (float)(((long long)k * kSample + L - 1) / L);
+  return (int)(e + 4.5f * sqrtf(e) + 4.f);
+}
+
+// Finds the digit that holds the kr-th largest of the counted keys (1 <= kr <= their number), how many keys of that
+// digit are needed and how many there are; clears the histogram.  All threads; two barriers.
+__device__ __forceinline__ void hist_find(SharedStream& sh, uint32_t kr) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint4* h4 = reinterpret_cast<uint4*>(sh.hist);
+  const uint4 c = h4[tid];                                   // digits 4 tid .. 4 tid + 3
+  h4[tid] = make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t s = c.x + c.y + c.z + c.w;
+  uint32_t incl = s;                                         // this lane and the lanes above it
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t n = __shfl_down_sync(0xffffffffu, incl, off);
+    if (lane + off < 32) incl += n;
+  }
+  if (lane == 0) sh.warp_tot[warp] = incl;
+  __syncthreads();
+  const uint32_t w = (lane < kSW && lane > warp) ? sh.warp_tot[lane] : 0u;
+  uint32_t gt = __reduce_add_sync(0xffffffffu, w) + incl - s;   // keys with a higher digit than this thread's
+  const uint32_t cc[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+  for (int d = 3; d >= 0; --d) {
+    const uint32_t ge = gt + cc[d];
+    if (gt < kr && kr <= ge) { sh.digit = 4 * tid + d; sh.rem = kr - gt; sh.n_eq = cc[d]; }   // exactly one digit
+    gt = ge;
+  }
+  __syncthreads();
+}
+
+// Key of the k-th largest key among those that visit(f) hands to f (key 0: not counted), resolved to its upper 22 bits
+// (kPasses = 2) or exactly (3); `need` of the `n_eq` keys equal to it belong to the k largest.  Needs a cleared histogram.
+template <int kPasses, typename Visit>
+__device__ __forceinline__ void kth_key(SharedStream& sh, uint32_t k, Visit visit, uint32_t& T, uint32_t& need, uint32_t& n_eq) {
+  uint32_t prefix = 0u, mask = 0u;
+#pragma unroll 1
+  for (int pass = 0; pass < kPasses; ++pass) {
+    const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
+    const uint32_t dm = pass == 2 ? 1023u : 2047u;
+    visit([&](uint32_t key) {
+      if (key != 0u && (key & mask) == prefix) atomicAdd(&sh.hist[(key >> shift) & dm], 1u);
+    });
+    __syncthreads();
+    hist_find(sh, k);
+    prefix |= sh.digit << shift;
+    mask |= dm << shift;
+    k = sh.rem;
+  }
+  T = prefix;
+  need = k;
+  n_eq = sh.n_eq;
+}
+
+// Exclusive block-wide scan; two barriers (the second keeps warp_tot stable until everyone has read it).
+__device__ __forceinline__ uint32_t stream_scan_excl(SharedStream& sh, uint32_t v) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t n = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += n;
+  }
+  if (lane == 31) sh.warp_tot[warp] = incl;
+  __syncthreads();
+  const uint32_t w = lane < warp ? sh.warp_tot[lane] : 0u;      // warp < kSW
+  const uint32_t base = __reduce_add_sync(0xffffffffu, w);
+  __syncthreads();
+  return base + incl - v;
+}
+
+__global__ void __launch_bounds__(kST, 2) topk_stream_kernel(const TopkParams p, int cap, int words) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  SharedStream& sh = *reinterpret_cast<SharedStream*>(smem_raw);
+  uint32_t* ckeys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(SharedStream));   // [cap] candidates; later the output
+  int* cidx = reinterpret_cast<int*>(ckeys + cap);                                  // [cap]
+  uint32_t* bm = reinterpret_cast<uint32_t*>(cidx + cap);                           // [words] one bit per key of the row
+  uint16_t* prefix16 = reinterpret_cast<uint16_t*>(sh.hist);                        // [words] during the write-out
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int L = p.L, n_sink = p.n_sink;
+  const int wpt = (words + kST - 1) / kST;                       // contiguous bitmap words per thread in the scans
+  auto set_bit = [&](int j) { atomicOr(&bm[j >> 5], 1u << (j & 31)); };
+
+#pragma unroll 1
+  for (long long row = blockIdx.x; row < p.rows; row += gridDim.x) {
+    const float* sc = p.scores + row * (long long)L;
+    int32_t* out = p.out + row * (long long)p.k_total;
+    const int k_row = p.k_rows != nullptr ? min(max(p.k_rows[row], n_sink), p.k_total) : p.k_total;
+    const int k = k_row - n_sink;
+    for (int i = tid; i < kDigits; i += kST) sh.hist[i] = 0u;
+    for (int i = tid; i < words; i += kST) bm[i] = 0u;
+    if (tid == 0) { sh.n_cand = 0u; sh.n_dead = 0u; sh.n_tie = 0u; }
+    __syncthreads();
+    if (tid < n_sink) set_bit(p.sinks[tid]);                     // until the end of the row: bit set == sink
+    __syncthreads();
+    auto is_sink = [&](int j) { return ((bm[j >> 5] >> (j & 31)) & 1u) != 0u; };
+
+    if (k > 0) {
+      // ---- 1. lower bound t: candidates are the keys above it (NaN included)
+      uint32_t t_key = 0u;
+      float t = -INFINITY;
+      const int r_s = sample_rank(k, L);
+      bool sampled = L > kSampleAll && r_s < kSample;
+      if (sampled) {
+        uint32_t s[kSample / kST];
+#pragma unroll
+        for (int u = 0; u < kSample / kST; ++u) s[u] = __float_as_uint(__ldg(sc + (int)(((long long)(u * kST + tid) * L) >> 12)));
+#pragma unroll
+        for (int u = 0; u < kSample / kST; ++u) {
+          const uint32_t key = score_key(__uint_as_float(s[u]));
+          s[u] = is_sink((int)(((long long)(u * kST + tid) * L) >> 12)) ? 2u : key;
+        }
+        uint32_t need, n_eq;
+        kth_key<2>(sh, (uint32_t)r_s, [&](auto f) {
+#pragma unroll
+          for (int u = 0; u < kSample / kST; ++u) f(s[u]);
+        }, t_key, need, n_eq);
+        t = __uint_as_float((t_key & 0x80000000u) ? (t_key & 0x7FFFFFFFu) : ~t_key);
+        if (t != t) { t = -INFINITY; sampled = false; }          // the bound fell among the NaNs: no bound
+      }
+      // ---- 2. one sweep over the row: aligned 16-byte loads (the row may start at any element; the chunks that reach
+      // beyond it are read element by element), the next kSU loads in flight while the current ones are processed
+      const int o = (int)((reinterpret_cast<uintptr_t>(sc) >> 2) & 3);
+      const int nch = (o + L + 3) >> 2;
+      auto load = [&](int c) -> float4 {
+        if (4 * c >= o && 4 * c + 4 <= o + L) return __ldcs(reinterpret_cast<const float4*>(sc - o) + c);
+        float4 f = make_float4(t, t, t, t);                      // t itself is no candidate
+        const int j = 4 * c - o;
+        if (j >= 0 && j < L) f.x = sc[j];
+        if (j + 1 >= 0 && j + 1 < L) f.y = sc[j + 1];
+        if (j + 2 >= 0 && j + 2 < L) f.z = sc[j + 2];
+        if (j + 3 >= 0 && j + 3 < L) f.w = sc[j + 3];
+        return f;
+      };
+      float4 nx[kSU];
+#pragma unroll
+      for (int u = 0; u < kSU; ++u) nx[u] = load(u * kST + tid);
+#pragma unroll 1
+      for (int c0 = 0; c0 < nch; c0 += kST * kSU) {
+        float4 v[kSU];
+#pragma unroll
+        for (int u = 0; u < kSU; ++u) v[u] = nx[u];
+        if (c0 + kST * kSU < nch) {
+#pragma unroll
+          for (int u = 0; u < kSU; ++u) nx[u] = load(c0 + kST * kSU + u * kST + tid);
+        }
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int u = 0; u < kSU; ++u)
+          cnt += (v[u].x <= t ? 0u : 1u) + (v[u].y <= t ? 0u : 1u) + (v[u].z <= t ? 0u : 1u) + (v[u].w <= t ? 0u : 1u);
+        uint32_t incl = cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const uint32_t n = __shfl_up_sync(0xffffffffu, incl, off);
+          if (lane >= off) incl += n;
+        }
+        uint32_t base = 0;
+        if (lane == 31) base = atomicAdd(&sh.n_cand, incl);
+        uint32_t pos = __shfl_sync(0xffffffffu, base, 31) + incl - cnt;
+        if (cnt != 0u && pos + cnt <= (uint32_t)cap) {           // (an overflow shows in n_cand)
+#pragma unroll
+          for (int u = 0; u < kSU; ++u) {
+            const int j = 4 * (c0 + u * kST + tid) - o;
+            const float f[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (!(f[e] <= t)) { ckeys[pos] = __float_as_uint(f[e]); cidx[pos] = j + e; ++pos; }
+          }
+        }
+      }
+      __syncthreads();
+      // ---- 3. the exact k-th key
+      const uint32_t C = sh.n_cand;
+      uint32_t T = 0u, need = 0u, n_eq = 0u;
+      bool from_row = false;
+      uint32_t live = 0;
+      if (C <= (uint32_t)cap) {
+        for (int i = tid; i < (int)C; i += kST) {                // sinks are no candidates; the others get their key
+          const bool sink = is_sink(cidx[i]);
+          ckeys[i] = sink ? 0u : score_key(__uint_as_float(ckeys[i]));
+          if (sink) atomicAdd(&sh.n_dead, 1u);
+        }
+        __syncthreads();
+        live = C - sh.n_dead;
+      }
+      auto row_key = [&](int j) { return is_sink(j) ? 0u : score_key(__ldg(sc + j)); };
+      auto visit_row = [&](auto f) { for (int j = tid; j < L; j += kST) f(row_key(j)); };
+      if (live >= (uint32_t)k) {
+        kth_key<3>(sh, (uint32_t)k, [&](auto f) { for (int i = tid; i < (int)C; i += kST) f(ckeys[i]); }, T, need, n_eq);
+      } else {
+        from_row = true;
+        bool tie = false;
+        if (sampled && C <= (uint32_t)cap) {
+          // a tie group on the bound itself (masses that underflow to zero): the k-th key is t
+          uint32_t n = 0;
+          visit_row([&](uint32_t key) { n += (key == t_key) ? 1u : 0u; });
+          n = __reduce_add_sync(0xffffffffu, n);
+          if (lane == 0) atomicAdd(&sh.n_tie, n);
+          __syncthreads();
+          n_eq = sh.n_tie;
+          tie = live + n_eq >= (uint32_t)k;
+          T = t_key;
+          need = (uint32_t)k - live;
+        }
+        if (!tie) kth_key<3>(sh, (uint32_t)k, visit_row, T, need, n_eq);
+      }
+      // ---- 4. bitmap of the selected keys: above T, and the `need` lowest indices among those equal to T
+      auto mark = [&](bool above, bool equal) {
+        if (from_row) {
+          // (keys of the row are compared without the sink test, whose bits may be gone: a sink belongs to the result)
+          for (int j = tid; j < L; j += kST) {
+            const uint32_t key = score_key(__ldg(sc + j));
+            if ((above && key > T) || (equal && key == T)) set_bit(j);
+          }
+        } else {
+          for (int i = tid; i < (int)C; i += kST) {
+            const uint32_t key = ckeys[i];
+            if ((above && key > T) || (equal && key == T)) set_bit(cidx[i]);
+          }
+        }
+      };
+      if (need == n_eq) {
+        mark(true, true);
+      } else {
+        __syncthreads();
+        for (int i = tid; i < words; i += kST) bm[i] = 0u;
+        __syncthreads();
+        mark(false, true);
+        __syncthreads();
+        if (from_row) {                                          // a sink that equals T takes no part in the ranking
+          if (tid < n_sink) atomicAnd(&bm[p.sinks[tid] >> 5], ~(1u << (p.sinks[tid] & 31)));
+          __syncthreads();
+        }
+        uint32_t n = 0;
+        for (int i = 0; i < wpt; ++i) { const int w = tid * wpt + i; if (w < words) n += __popc(bm[w]); }
+        uint32_t before = stream_scan_excl(sh, n);
+        for (int i = 0; i < wpt; ++i) {
+          const int w = tid * wpt + i;
+          if (w >= words) break;
+          uint32_t b = bm[w];
+          const uint32_t c = __popc(b);
+          uint32_t keep = before >= need ? 0u : min(need - before, c);
+          uint32_t r = 0u;
+          for (; keep > 0u; --keep) { const uint32_t low = b & (0u - b); r |= low; b ^= low; }
+          bm[w] = r;
+          before += c;
+        }
+        __syncthreads();
+        mark(true, false);
+        if (tid < n_sink) set_bit(p.sinks[tid]);
+      }
+      __syncthreads();
+    }
+    // ---- 5. write-out: output position of every bitmap word's first bit, then one word per lane, staged so that the
+    // global stores are consecutive
+    {
+      uint32_t n = 0;
+      for (int i = 0; i < wpt; ++i) { const int w = tid * wpt + i; if (w < words) n += __popc(bm[w]); }
+      uint32_t before = stream_scan_excl(sh, n);
+      for (int i = 0; i < wpt; ++i) {
+        const int w = tid * wpt + i;
+        if (w >= words) break;
+        prefix16[w] = (uint16_t)before;
+        before += __popc(bm[w]);
+      }
+      __syncthreads();
+      for (int w = tid; w < words; w += kST) {
+        uint32_t b = bm[w];
+        int pos = prefix16[w];
+        while (b != 0u) {
+          if (pos < k_row) ckeys[pos] = (uint32_t)(w * 32 + __ffs((int)b) - 1);
+          ++pos;
+          b &= b - 1u;
+        }
+      }
+      __syncthreads();
+      for (int i = tid; i < p.k_total; i += kST) out[i] = i < k_row ? (int)ckeys[i] : 0;   // beyond the row's budget: padding
+    }
+  }
+}
+
 }  // namespace
+
+constexpr size_t kStreamSmemLimit = 112 * 1024;   // two CTAs per SM
 
 size_t topk_stage_limit_bytes() { return 200 * 1024; }
 
 int launch_topk_select(const TopkParams& p, cudaStream_t stream) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // streaming path: whenever the candidates that the sampled bound lets through fit in shared memory beside the bitmap
+  if (p.L <= kStreamMaxL) {
+    const int k = p.k_total - p.n_sink;
+    const bool all = p.L <= kSampleAll;
+    const int r_s = sample_rank(k > 0 ? k : 1, p.L);
+    long long cap = p.L;
+    if (!all) {
+      // five standard deviations above the expected number, and 6% for the bound's truncation to 22 bits
+      const double c = (r_s + 5.0 * sqrt((double)r_s) + 8.0) * p.L / kSample * 1.06 + 64.0;
+      cap = (long long)c < p.L ? (long long)c : p.L;
+    }
+    cap = (cap + 3) & ~3ll;
+    const int words = (p.L + 31) / 32;
+    const size_t smem = sizeof(SharedStream) + (size_t)cap * 8 + (size_t)words * 4;
+    if ((all || r_s < kSample) && smem <= kStreamSmemLimit) {
+      if (cudaFuncSetAttribute(topk_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -8;
+      const long long slots = 2ll * sms;
+      topk_stream_kernel<<<(unsigned)(p.rows < slots ? p.rows : slots), kST, smem, stream>>>(p, (int)cap, words);
+      return cudaGetLastError() == cudaSuccess ? 0 : -8;
+    }
+  }
   if (p.L <= kKpt * kRT) {
     // register-resident path; cp.async needs every row start 16-byte aligned
     const size_t smem = sizeof(SharedReg) + (size_t)kCandCap * 4 + (size_t)kKpt * kRT * 4;

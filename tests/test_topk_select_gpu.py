@@ -78,3 +78,32 @@ def test_register_path_structured_rows(cuda_device, L):
     out = _run(cuda_device, scores, k_total, [(0, 4)])
     ref = select_topk_ref(scores, k_total, sinks=range(4))
     assert torch.equal(out, ref)
+
+
+# rows around the streaming kernel's edges: every key a candidate / sampled bound (8,192), unaligned row starts (odd
+# lengths), 16-bit word prefixes (131,072), budgets at which another kernel takes over
+@pytest.mark.parametrize("L,k_total", [(130, 128), (8192, 2048), (8193, 2048), (16381, 9000), (33001, 128), (40000, 20000),
+                                       (98279, 4096), (131072, 8192), (131073, 512)])
+def test_streaming_edges(cuda_device, L, k_total):
+    g = torch.Generator().manual_seed(L)
+    k_total = min(k_total, L)
+    rows = [torch.rand(L, generator=g) ** 12, torch.randn(L, generator=g)]
+    under = torch.rand(L, generator=g)                                     # fewer than k masses survive, the rest tie at zero
+    under[torch.randperm(L, generator=g)[: L - k_total // 2]] = 0.0
+    rows.append(under)
+    rows.append(torch.arange(L).float().flip(0))                           # winners in front
+    spike = torch.full((L,), -float("inf"))                                # fewer than k finite keys
+    spike[::7] = torch.rand(spike[::7].numel(), generator=g)
+    rows.append(spike)
+    nan_row = torch.rand(L, generator=g)
+    nan_row[torch.randperm(L, generator=g)[: L // 2]] = float("nan")
+    rows.append(nan_row)
+    rows.append(torch.randint(0, 40, (L,), generator=g).float())           # a tie group around rank k
+    scores = torch.stack(rows)
+    sinks = [0, 1, 2, 3, L - 1]
+    ranges = [(0, 4), (L - 1, L)]
+    ref = select_topk_ref(scores, k_total, sinks=sinks)
+    assert torch.equal(_run(cuda_device, scores, k_total, ranges), ref)
+    shifted = torch.empty(scores.numel() + 1, device=cuda_device)[1:].view(scores.shape)   # 4-byte aligned base
+    shifted.copy_(scores)
+    assert torch.equal(_run(cuda_device, shifted, k_total, ranges), ref)

@@ -7,18 +7,15 @@
 // by their projection on that direction and is split at the block-aligned midpoint.
 //
 // Per level, with no host synchronisation anywhere (the tree shape depends only on N and C):
-//   gram     tcgen05: G += X_tile^T X_tile over 128-row tiles gathered through the current
-//            permutation.  The SAME shared-memory tile serves as both MMA operands (MN-major A and
-//            MN-major B); a second, 16-column MMA against a tile of ones yields the column sums s.
-//            Big nodes are split into chunks of 2048 rows whose partial results are summed in a
-//            fixed order by the next kernel (deterministic, no atomics).
-//   power    one CTA per node: reduce partials, centre, normalise the start vector, iterate.
-//   project  a = x . v in fp32 per row (one warp per row), emitted as 64-bit sort keys
-//            (order-preserving float bits << 32 | position inside the node): unique keys, so the
-//            sort is stable by construction; the fp32 projections can be dumped for checking.
-//   sort     bitonic network over power-of-two padded segments: shared-memory stages, plus
-//            global compare-exchange steps when a segment exceeds one CTA's tile.
-//   scatter  new order written back through the sorted positions.
+//   node     tcgen05: G += X_tile^T X_tile over 128-row tiles gathered through the current permutation.  The SAME
+//            shared-memory tile serves as both MMA operands (MN-major A and MN-major B); a second, 16-column MMA
+//            against a tile of ones yields the column sums s.  A node of up to 2048 rows is finished by its CTA: centre,
+//            normalise the start vector, iterate, project its rows (fp32), emit 64-bit sort keys (order-preserving
+//            float bits << 32 | position inside the node: unique keys, so the sort is stable by construction).
+//   power, project   the same for nodes of several 2048-row items, whose partial sums are added in a fixed order
+//            (deterministic, no atomics).
+//   sort     bitonic network over power-of-two padded segments, out of registers; global compare-exchange steps when a
+//            segment exceeds one CTA's tile.  The last kernel writes the new order.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -75,29 +72,66 @@ struct LevelTables {
   int* item_row0;    // [items] first row (relative to node start)
 };
 
-__global__ void pddp_tables_kernel(int N, int C, int* tab, int max_levels, int stride) {
-  // single thread: fills, for every level, node_start/node_size/node_item0/item_node/item_row0
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One CTA; a level's intervals are handled 1,024 at a time, with one scan for the positions of their work items and of
+// their children (a single thread walking the lists took 73 us for 256 blocks).
+constexpr int kTableThreads = 1024;
+__global__ void __launch_bounds__(kTableThreads) pddp_tables_kernel(int N, int C, int* tab, int max_levels, int stride) {
+  __shared__ unsigned long long warp_tot[kTableThreads / 32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int K = (N + C - 1) / C;
   // two scratch interval lists live at the end of the table area
   int* lo = tab + (size_t)max_levels * stride;
   int* hi = lo + kMaxNodes;
   int* lo2 = hi + kMaxNodes;
   int* hi2 = lo2 + kMaxNodes;
-  int n = 1; lo[0] = 0; hi[0] = K;
-  for (int lv = 0; lv < max_levels && any_splittable(lo, hi, n); ++lv) {
+  if (tid == 0) { lo[0] = 0; hi[0] = K; }
+  __syncthreads();
+  int n = 1;
+  for (int lv = 0; lv < max_levels; ++lv) {
     int* t = tab + (size_t)lv * stride;
     int* node_start = t, *node_size = t + kMaxNodes, *node_item0 = t + 2 * kMaxNodes;
     int* item_node = t + 3 * kMaxNodes, *item_row0 = item_node + (stride - 3 * kMaxNodes) / 2;
-    int items = 0;
-    for (int i = 0; i < n; ++i) {
-      const int s = lo[i] * C, e = min(hi[i] * C, N);
-      node_start[i] = s; node_size[i] = e - s; node_item0[i] = items;
-      for (int r = 0; r < e - s; r += kChunkRows) { item_node[items] = i; item_row0[items] = r; ++items; }
+    unsigned long long run = 0ull;                       // (work items << 32 | children) of the intervals before this batch
+    for (int i0 = 0; i0 < n; i0 += kTableThreads) {
+      const int i = i0 + tid;
+      int l = 0, h = 0, size = 0;
+      unsigned long long v = 0ull;
+      if (i < n) {
+        l = lo[i]; h = hi[i];
+        size = min(h * C, N) - l * C;
+        v = ((unsigned long long)((size + kChunkRows - 1) / kChunkRows) << 32) | (h - l > 1 ? 2u : 1u);
+      }
+      unsigned long long incl = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long m = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += m;
+      }
+      if (lane == 31) warp_tot[warp] = incl;
+      __syncthreads();
+      unsigned long long before = run, all = run;
+      for (int w = 0; w < kTableThreads / 32; ++w) {
+        if (w < warp) before += warp_tot[w];
+        all += warp_tot[w];
+      }
+      before += incl - v;
+      if (i < n) {
+        const int item0 = (int)(before >> 32), c0 = (int)(before & 0xFFFFFFFFull);
+        node_start[i] = l * C; node_size[i] = size; node_item0[i] = item0;
+        for (int r = 0, it = item0; r < size; r += kChunkRows, ++it) { item_node[it] = i; item_row0[it] = r; }
+        if (h - l > 1) {
+          const int mid = l + (h - l) / 2;
+          lo2[c0] = l; hi2[c0] = mid; lo2[c0 + 1] = mid; hi2[c0 + 1] = h;
+        } else {
+          lo2[c0] = l; hi2[c0] = h;
+        }
+      }
+      run = all;
+      __syncthreads();
     }
-    const int m = split_level(lo, hi, n, lo2, hi2);
-    for (int i = 0; i < m; ++i) { lo[i] = lo2[i]; hi[i] = hi2[i]; }
-    n = m;
+    n = (int)(run & 0xFFFFFFFFull);
+    int* x = lo; lo = lo2; lo2 = x;
+    x = hi; hi = hi2; hi2 = x;
   }
 }
 
@@ -113,42 +147,176 @@ __device__ __forceinline__ uint32_t swz(int row, int c) {
   return static_cast<uint32_t>((c >> 3) * 16384 + row * 128 + (((c & 7) ^ (row & 7)) << 4));
 }
 
-// ------------------------------------------------------------------------------------------
-// gram: partial[bh][item] = (G 128x128, s 128) over the item's rows
-// ------------------------------------------------------------------------------------------
-constexpr int kGramThreads = 160;       // 4 load/epilogue warps + 1 MMA warp
-constexpr int kGramSmem = 2 * 32768 + 16384 + 256 + 1024;
+__device__ __forceinline__ uint32_t float_key(float f) {
+  uint32_t u = __float_as_uint(f);
+  if (f == 0.f) u = 0u;                                        // -0 == +0
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+constexpr int kProjRows = 8;            // (wide path) rows per warp: eight independent row loads in flight per lane
+constexpr int kNodeThreads = 160;       // 4 gather / epilogue warps + 1 MMA warp
+constexpr int kBufs = 3;                // 128-row tiles in flight per CTA
+constexpr int kTileBytes = 32768;
 constexpr int kPartialFloats = 128 * 128 + 128;
 
-template <bool kFp16>
-__global__ void __launch_bounds__(kGramThreads, 1) pddp_gram_kernel(PddpParams p, int lv, const int* perm_in) {
+struct NodeSmem {
+  static constexpr int kOnes = kBufs * kTileBytes;             // 16 rows x 128 B of ones
+  static constexpr int kVec = kOnes + 2048;                    // float [128]
+  static constexpr int kSum = kVec + 512;                      // float [128]
+  static constexpr int kRed = kSum + 512;                      // float [4]
+  static constexpr int kBars = kRed + 16;                      // kBufs full, kBufs empty, done, drain
+  static constexpr int kSlot = kBars + (2 * kBufs + 2) * 8;
+  static constexpr int kDynamic = kSlot + 16 + 1024;
+};
+
+// One warp copies rows 32 * warp .. + 31 of a tile of gathered rows; lane l holds the source row of tile row
+// 32 * warp + l (negative: zero row).  D / 8 lanes cover one row, so every request is whole rows.
+template <int D>
+__device__ __forceinline__ void gather_tile_rows(uint32_t tile, int warp, int lane, int my_id, const uint8_t* xb, size_t row_bytes) {
+  constexpr int kChunks = D / 8, kRpi = 32 / kChunks;
+  const int sub = lane / kChunks, c = lane % kChunks;
+#pragma unroll
+  for (int i = 0; i < 32 / kRpi; ++i) {
+    const int rl = i * kRpi + sub;
+    const int id = __shfl_sync(0xffffffffu, my_id, rl);
+    const uint32_t dst = tile + swz(warp * 32 + rl, c);
+    if (id >= 0) cp_async16(dst, xb + (size_t)id * row_bytes + c * 16);
+    else cp_async16_zfill(dst, xb, 0);
+  }
+}
+
+// fp32 projection of tile row `row` on vec.  The additions are those of a warp that holds four elements per lane and
+// reduces by butterflies from distance 16 down: element group l with group l + 16 first, then + 8, + 4, + 2, + 1.
+template <int D, bool kFp16>
+__device__ __forceinline__ float project_row(uint32_t tile, int row, const float* vec) {
+  auto quad = [&](uint32_t w0, uint32_t w1, const float4 v) {
+    float2 a, b;
+    if (kFp16) {
+      a = __half22float2(*reinterpret_cast<const __half2*>(&w0));
+      b = __half22float2(*reinterpret_cast<const __half2*>(&w1));
+    } else {
+      a = make_float2(bf16_lo(w0), bf16_hi(w0));
+      b = make_float2(bf16_lo(w1), bf16_hi(w1));
+    }
+    return fmaf(a.x, v.x, fmaf(a.y, v.y, fmaf(b.x, v.z, b.y * v.w)));
+  };
+  const float4* v4 = reinterpret_cast<const float4*>(vec);
+  float s[16];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint4 w = lds_v4(tile + swz(row, c));
+    s[2 * c] = quad(w.x, w.y, v4[2 * c]);
+    s[2 * c + 1] = quad(w.z, w.w, v4[2 * c + 1]);
+    if (D == 128) {
+      const uint4 u = lds_v4(tile + swz(row, c + 8));
+      s[2 * c] += quad(u.x, u.y, v4[2 * c + 16]);
+      s[2 * c + 1] += quad(u.z, u.w, v4[2 * c + 17]);
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int l = 0; l < o; ++l) s[l] += s[l + o];
+  return s[0];
+}
+
+// Projects `rows` gathered rows (positions pos0 .. of head bh, which are r_first .. of their node) on vec and writes
+// their sort keys.  128 threads, thread == row of a tile; a warp consumes only rows that it gathered itself, so the tiles
+// need no barrier.  With `resident`, tile t already lies in buffer t.
+template <int D, bool kFp16>
+__device__ __forceinline__ void project_rows(uint32_t s_base, int warp, int lane, const uint8_t* xb, size_t row_bytes, const int* ids,
+                                             int rows, int r_first, const float* vec, unsigned long long* keys, float* proj_out,
+                                             bool resident) {
+  const int n_tiles = (rows + 127) / 128, mine = warp * 32 + lane;
+  auto load_id = [&](int t) { const int r = t * 128 + mine; return r < rows ? ids[r] : -1; };
+  int id_next = 0;
+  if (!resident) {
+#pragma unroll
+    for (int t = 0; t < kBufs - 1; ++t) {
+      if (t < n_tiles) gather_tile_rows<D>(s_base + t * kTileBytes, warp, lane, load_id(t), xb, row_bytes);
+      cp_async_commit_group();
+    }
+    id_next = load_id(kBufs - 1);
+  }
+  int buf = 0, fill = kBufs - 1;
+#pragma unroll 1
+  for (int t = 0; t < n_tiles; ++t) {
+    if (!resident) {
+      // tile t + kBufs - 1 goes where tile t - 1 was (read by this warp alone, one iteration ago)
+      if (t + kBufs - 1 < n_tiles) gather_tile_rows<D>(s_base + fill * kTileBytes, warp, lane, id_next, xb, row_bytes);
+      cp_async_commit_group();
+      id_next = load_id(t + kBufs);
+      cp_async_wait_group<kBufs - 1>();
+      __syncwarp();
+    }
+    const float a = project_row<D, kFp16>(s_base + buf * kTileBytes, mine, vec);
+    const int r = t * 128 + mine;
+    if (r < rows) {
+      keys[r_first + r] = ((unsigned long long)float_key(a) << 32) | (unsigned)(r_first + r);
+      if (proj_out != nullptr) proj_out[r] = a;
+    }
+    __syncwarp();
+    buf = buf + 1 == kBufs ? 0 : buf + 1;
+    fill = fill + 1 == kBufs ? 0 : fill + 1;
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// node: Gram matrix of an item's rows; for a node that is one item also its principal direction and its sort keys
+//
+// Bound by the gathered reads of X (whole rows, 16 or 8 lanes each, kBufs tiles in flight per CTA and two CTAs per SM).
+// A node of one item (up to kChunkRows rows: half of the levels and most of the nodes) never leaves its CTA: the Gram
+// matrix stays in tensor memory, thread d holds row d, the power iterations are dot products of that row with a vector
+// in shared memory, and the projections read the tiles that are still in shared memory (nodes of up to kBufs tiles) or
+// gather them again out of L2.  Larger nodes write their partial sums for the power kernel; G is symmetric, so thread d
+// writes column d and every store is one 128-byte line per warp.
+// Same sums in the same order as a kernel per stage had: identical permutations.
+// Measured (24 heads x 32,760 tokens x 128, 8 levels, kernel times of one call): Gram 1,140 + power 638 + project 556 us
+// before; node 599 + power 62 + project 196 us now (X read twice per level at the measured copy rate: 490 us).  Of that,
+// lanes that load whole rows instead of a row each, the transposed partial store and the fused power step are the most.
+// ------------------------------------------------------------------------------------------
+template <int D, bool kFp16>
+__global__ void __launch_bounds__(kNodeThreads, 2) pddp_node_kernel(PddpParams p, int lv, int nodes, int pad, const int* perm_in,
+                                                                    const float* v0, float* proj_out) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  using S = NodeSmem;
   const uint32_t s_base = smem_u32(smem);
-  const uint32_t sOnes = s_base + 65536;
-  const uint32_t bars = s_base + 65536 + 16384;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 65536 + 16384 + 128);
-  auto bar = [&](int i) { return bars + 8u * i; };   // 0,1 full; 2,3 empty; 4 done
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t sOnes = s_base + S::kOnes;
+  const uint32_t bars = s_base + S::kBars;
+  float* vec = reinterpret_cast<float*>(smem + S::kVec);
+  float* ssum = reinterpret_cast<float*>(smem + S::kSum);
+  float* red = reinterpret_cast<float*>(smem + S::kRed);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + S::kSlot);
+  enum { FULL = 0, EMPTY = kBufs, DONE = 2 * kBufs };
+  auto bar = [&](int i) { return bars + 8u * i; };
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const LevelTables T = level_tables(p.tables, lv, p.table_stride);
   const int item = blockIdx.x, bh = blockIdx.y;
   const int node = T.item_node[item];
   const int row_begin = T.item_row0[item];
-  const int rows = min(kChunkRows, T.node_size[node] - row_begin);
+  const int size = T.node_size[node];
+  const int rows = min(kChunkRows, size - row_begin);
   const int pos0 = T.node_start[node] + row_begin;
   const int n_tiles = (rows + 127) / 128;
-  const int D = p.D;
 
   if (tid == 0) {
-    mbar_init(bar(0), 128); mbar_init(bar(1), 128); mbar_init(bar(2), 1); mbar_init(bar(3), 1); mbar_init(bar(4), 1);
+    for (int i = 0; i < kBufs; ++i) { mbar_init(bar(FULL + i), 128); mbar_init(bar(EMPTY + i), 1); }
+    mbar_init(bar(DONE), 1);
     mbar_fence_init();
   }
   if (warp == 4) { tmem_alloc(smem_u32(tmem_slot), 256); tmem_relinquish(); }
   // ones tile: rows 0..15 (N = 16), 16 K-columns of 1.0 (K-major, 128-byte swizzled rows)
   if (tid < 16) {
     const uint32_t one2 = kFp16 ? 0x3C003C00u : 0x3F803F80u;
-    *reinterpret_cast<uint4*>(smem + 65536 + swz(tid, 0)) = make_uint4(one2, one2, one2, one2);
-    *reinterpret_cast<uint4*>(smem + 65536 + swz(tid, 1)) = make_uint4(one2, one2, one2, one2);
+    *reinterpret_cast<uint4*>(smem + S::kOnes + swz(tid, 0)) = make_uint4(one2, one2, one2, one2);
+    *reinterpret_cast<uint4*>(smem + S::kOnes + swz(tid, 1)) = make_uint4(one2, one2, one2, one2);
+  }
+  if (D == 64) {
+    // features 64..127 of the 128-wide product do not exist: their column block is zero once and for all
+    for (int i = tid; i < kBufs * 1024; i += kNodeThreads)
+      *reinterpret_cast<uint4*>(smem + (i >> 10) * kTileBytes + 16384 + (i & 1023) * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   fence_proxy_async_smem();
   tc_fence_before();
@@ -158,72 +326,135 @@ __global__ void __launch_bounds__(kGramThreads, 1) pddp_gram_kernel(PddpParams p
 
   if (warp < 4) {
     // ---- gather rows of each tile through the permutation
-    const int chunks = D / 8;                    // 16-byte chunks per row (8 or 16)
     const uint8_t* xb = reinterpret_cast<const uint8_t*>(p.x) + 2 * (size_t)bh * p.x_stride_bh;
     const size_t row_bytes = 2 * (size_t)p.x_stride_row;
+    const int* ids = perm_in + (size_t)bh * p.N + pos0;
     bool ok = true;
-    for (int t = 0; t < n_tiles && ok; ++t) {
-      const int buf = t & 1;
-      if (t >= 2) ok = mbar_wait(bar(2 + buf), ((t >> 1) - 1) & 1, p.status, 60);
-      if (!ok) break;
-      const int r = t * 128 + tid;               // row of the item handled by this thread
-      const uint8_t* src = nullptr;
-      if (r < rows) src = xb + (size_t)perm_in[(size_t)bh * p.N + pos0 + r] * row_bytes;
-      const uint32_t dst = s_base + buf * 32768;
-#pragma unroll 4
-      for (int c = 0; c < 16; ++c) {
-        if (src != nullptr && c < chunks) cp_async16(dst + swz(tid, c), src + c * 16);
-        else cp_async16_zfill(dst + swz(tid, c), xb, 0);
+    {
+      int id_next = tid < rows ? ids[tid] : -1;
+      int buf = 0, phase = 0;
+#pragma unroll 1
+      for (int t = 0; t < n_tiles && ok; ++t) {
+        const int id = id_next, r1 = (t + 1) * 128 + tid;
+        id_next = r1 < rows ? ids[r1] : -1;
+        if (t >= kBufs) ok = mbar_wait(bar(EMPTY + buf), phase ^ 1, p.status, 60);
+        if (!ok) break;
+        gather_tile_rows<D>(s_base + buf * kTileBytes, warp, lane, id, xb, row_bytes);
+        cp_async_arrive_noinc(bar(FULL + buf));
+        if (++buf == kBufs) { buf = 0; phase ^= 1; }
       }
-      cp_async_arrive_noinc(bar(buf));
     }
     cp_async_wait_all();
-    // ---- epilogue: thread d owns feature row d of G (TMEM lane d)
-    if (ok) ok = mbar_wait(bar(4), 0, p.status, 61);
+    if (ok) ok = mbar_wait(bar(DONE), 0, p.status, 61);
+    // (the four warps agree, so that none waits at the named barriers below for one that has given up)
+    ok = !named_bar_red_or(1, 128, !ok);
     if (ok) {
       tc_fence_after();
-      float* out = p.partial + ((size_t)bh * p.max_items + item) * kPartialFloats;
+      const int d = tid;                                       // feature row of G == TMEM lane
       const uint32_t lane_addr = (static_cast<uint32_t>(warp) * 32u) << 16;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        tmem_ld32(tmem + lane_addr + c * 32, r);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) out[(size_t)tid * 128 + c * 32 + i] = __uint_as_float(r[i]);
-      }
       uint32_t r8[8];
       tmem_ld8(tmem + lane_addr + 128, r8);
       tmem_wait_ld();
-      out[128 * 128 + tid] = __uint_as_float(r8[0]);
+      const float s_d = __uint_as_float(r8[0]);
+      if (size > kChunkRows) {
+        float* out = p.partial + ((size_t)bh * p.max_items + item) * kPartialFloats;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem + lane_addr + c * 32, r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) out[(size_t)(c * 32 + i) * 128 + d] = __uint_as_float(r[i]);
+        }
+        out[128 * 128 + d] = s_d;
+      } else {
+        // ---- centred Gram matrix, back in tensor memory
+        ssum[d] = s_d;
+        named_bar_sync(1, 128);
+        const float inv_n = 1.f / (float)size;
+#pragma unroll 1
+        for (int c = 0; c < D / 8; ++c) {
+          tmem_ld8(tmem + lane_addr + c * 8, r8);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) r8[i] = __float_as_uint(__uint_as_float(r8[i]) - ssum[c * 8 + i] * s_d * inv_n);
+          tmem_st8(tmem + lane_addr + c * 8, r8);
+        }
+        tmem_wait_st();
+        // ---- power iterations
+        auto sum_128 = [&](float x) {
+          for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+          if (lane == 0) red[warp] = x;
+          named_bar_sync(1, 128);
+          return (red[0] + red[1]) + (red[2] + red[3]);
+        };
+        float v = d < D ? v0[((size_t)bh * nodes + node) * D + d] : 0.f;
+        float nrm = sqrtf(sum_128(v * v));
+        v /= fmaxf(nrm, 1e-12f);
+        for (int iter = 0; iter < p.pow_iters; ++iter) {
+          vec[d] = v;
+          named_bar_sync(1, 128);
+          float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+          for (int c = 0; c < D / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld32(tmem + lane_addr + c * 32, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 x = reinterpret_cast<const float4*>(vec)[c * 8 + i];
+              a[0] += __uint_as_float(r[4 * i]) * x.x;
+              a[1] += __uint_as_float(r[4 * i + 1]) * x.y;
+              a[2] += __uint_as_float(r[4 * i + 2]) * x.z;
+              a[3] += __uint_as_float(r[4 * i + 3]) * x.w;
+            }
+          }
+          v = (a[0] + a[1]) + (a[2] + a[3]);
+          nrm = sqrtf(sum_128(v * v));
+          v /= fmaxf(nrm, 1e-12f);
+        }
+        vec[d] = v;                                            // (every thread is past its last read: sum_128's barrier)
+        named_bar_sync(1, 128);
+        // ---- projections and sort keys; slots beyond the node sort last
+        unsigned long long* keys = p.keys + (size_t)bh * p.key_stride + (size_t)node * pad;
+        project_rows<D, kFp16>(s_base, warp, lane, xb, row_bytes, ids, rows, 0, vec, keys,
+                               proj_out != nullptr ? proj_out + (size_t)bh * p.N + pos0 : nullptr, n_tiles <= kBufs);
+        for (int r = rows + tid; r < pad; r += 128) keys[r] = 0xFFFFFFFFFFFFFFFFull;
+        cp_async_wait_all();
+      }
     }
     tc_fence_before();
   } else {
-    if (lane == 0) {
+    {
       constexpr uint32_t kFmt = kFp16 ? 0u : 1u;
       constexpr uint32_t idesc_g = mma_idesc(kFmt, kFmt, 1, 1, 128, 128);   // A and B both MN-major
       constexpr uint32_t idesc_s = mma_idesc(kFmt, kFmt, 1, 0, 128, 16);    // B = ones, K-major
       constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
       auto desc = [&](uint32_t lo) { return (static_cast<uint64_t>(kDescHi) << 32) | lo; };
       const uint32_t ones_lo = ((sOnes & 0x3FFFFu) >> 4) | (1u << 16);
+      const bool leader = elect_one();
       bool ok = true;
+      int buf = 0, phase = 0;
+#pragma unroll 1
       for (int t = 0; t < n_tiles && ok; ++t) {
-        const int buf = t & 1;
-        ok = mbar_wait(bar(buf), (t >> 1) & 1, p.status, 62);
+        ok = mbar_wait(bar(FULL + buf), phase, p.status, 62);
         if (!ok) break;
         fence_proxy_async_smem();
         tc_fence_after();
-        const uint32_t xlo = (((s_base + buf * 32768) & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16);
+        const uint32_t xlo = (((s_base + buf * kTileBytes) & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {             // 16 rows per k-step
           const uint64_t dx = desc(xlo + j * (2048 >> 4));
-          mma_f16_ss(tmem, dx, dx, idesc_g, (t > 0) || (j > 0));
-          mma_f16_ss(tmem + 128, dx, desc(ones_lo), idesc_s, (t > 0) || (j > 0));
+          if (leader) {
+            mma_f16_ss(tmem, dx, dx, idesc_g, (t > 0) || (j > 0));
+            mma_f16_ss(tmem + 128, dx, desc(ones_lo), idesc_s, (t > 0) || (j > 0));
+          }
         }
-        tc_commit(bar(2 + buf));
+        if (leader) tc_commit(bar(EMPTY + buf));
+        if (++buf == kBufs) { buf = 0; phase ^= 1; }
       }
-      if (ok) tc_commit(bar(4));
-      else { tc_commit(bar(4)); mbar_wait_quiet(bar(4), 0, 1 << 20); }
+      if (leader) tc_commit(bar(DONE));
+      if (!ok) mbar_wait_quiet(bar(DONE), 0, 1 << 20);     // outstanding products retire before tensor memory is released
     }
     __syncwarp();
     tc_fence_before();
@@ -233,14 +464,13 @@ __global__ void __launch_bounds__(kGramThreads, 1) pddp_gram_kernel(PddpParams p
 }
 
 // ------------------------------------------------------------------------------------------
-// power: v[bh][node] = principal direction of the node (pow_iters normalised mat-vecs)
+// power: dir[bh][node] = principal direction of a node of several items (pow_iters normalised mat-vecs)
 // ------------------------------------------------------------------------------------------
 
-// 512 threads: thread (d, q) = (tid & 127, tid >> 7) owns element d and the Gram rows e = q (mod 4).  The
-// arithmetic is exactly that of a 128-thread version with four accumulators per element (a_q summed over
-// e = q, q+4, ... in increasing order, combined as (a0 + a1) + (a2 + a3)), so results do not depend on the
-// thread count; four times the threads only shorten the dependent load and FMA chains, which is what the
-// deep levels with thousands of small nodes are bound by.
+// 512 threads: thread (d, q) = (tid & 127, tid >> 7) owns element d and the Gram rows e = q (mod 4); accumulators a_q
+// over e = q, q+4, ... in increasing order, combined as (a0 + a1) + (a2 + a3).  A level has only 1 to 8 such nodes per
+// head: the kernel is bound by the latency of summing the partials, so eight elements of a chunk and several chunks
+// are loaded at once.
 __global__ void __launch_bounds__(512, 1) pddp_power_kernel(PddpParams p, int lv, int nodes, const float* v0) {
   extern __shared__ __align__(16) float sm[];
   float* G = sm;                 // 128 x 128, symmetric
@@ -250,19 +480,27 @@ __global__ void __launch_bounds__(512, 1) pddp_power_kernel(PddpParams p, int lv
   const LevelTables T = level_tables(p.tables, lv, p.table_stride);
   const int node = blockIdx.x, bh = blockIdx.y, d = threadIdx.x & 127, q = threadIdx.x >> 7;
   const int size = T.node_size[node];
+  if (size <= kChunkRows) return;                              // done by the node kernel
   const int item0 = T.node_item0[node];
   const int n_items = (size + kChunkRows - 1) / kChunkRows;
   const float* part = p.partial + ((size_t)bh * p.max_items + item0) * kPartialFloats;
   // fixed-order reduction of the partial Gram matrices
   float s_d = 0.f;
+#pragma unroll 8
   for (int it = 0; it < n_items; ++it) s_d += part[(size_t)it * kPartialFloats + 128 * 128 + d];
   if (q == 0) vec[d] = s_d;
   __syncthreads();
   const float inv_n = 1.f / (float)size;
-  for (int e = q; e < 128; e += 4) {
-    float g = 0.f;
-    for (int it = 0; it < n_items; ++it) g += part[(size_t)it * kPartialFloats + (size_t)e * 128 + d];   // G[e][d], coalesced
-    G[e * 128 + d] = g - vec[e] * s_d * inv_n;
+#pragma unroll 1
+  for (int e0 = q; e0 < 128; e0 += 32) {
+    float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int it = 0; it < n_items; ++it) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] += part[(size_t)it * kPartialFloats + (size_t)(e0 + 4 * j) * 128 + d];   // G[e][d], coalesced
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) G[(e0 + 4 * j) * 128 + d] = g[j] - vec[e0 + 4 * j] * s_d * inv_n;
   }
   __syncthreads();
   // sum over the 128 elements, identical in all four thread groups: warp sums, then (r0 + r1) + (r2 + r3)
@@ -294,72 +532,28 @@ __global__ void __launch_bounds__(512, 1) pddp_power_kernel(PddpParams p, int lv
 }
 
 // ------------------------------------------------------------------------------------------
-// project: fp32 projection of every row on its node's direction -> 64-bit sort keys
+// project: sort keys of the items of nodes that are more than one item
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t float_key(float f) {
-  uint32_t u = __float_as_uint(f);
-  if (f == 0.f) u = 0u;                                        // -0 == +0
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-constexpr int kProjRows = 8;     // rows per warp: eight independent row loads in flight per lane
-
-template <bool kFp16>
-__global__ void __launch_bounds__(256) pddp_project_kernel(PddpParams p, int lv, int nodes, int pad, const int* perm_in,
-                                                           float* proj_out) {
+template <int D, bool kFp16>
+__global__ void __launch_bounds__(128) pddp_project_kernel(PddpParams p, int lv, int pad, const int* perm_in, float* proj_out) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ float vec[128];
   const LevelTables T = level_tables(p.tables, lv, p.table_stride);
-  const int bh = blockIdx.y;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  // one warp per kProjRows consecutive slots of the padded key array (slot = node * pad + r); pad is a
-  // multiple of kProjRows, so the slots of a warp belong to one node
-  const long long total = (long long)nodes * pad;
-  const long long slot0 = warp * kProjRows;
-  if (slot0 >= total) return;
-  const int node = (int)(slot0 / pad), r0 = (int)(slot0 % pad);
-  unsigned long long* keys = p.keys + (size_t)bh * p.key_stride;
-  const int nsize = T.node_size[node];
-  const int pos0 = T.node_start[node] + r0;
-  const bool lane_live = lane * 4 < p.D;
-  float4 vv = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (lane_live) vv = *reinterpret_cast<const float4*>(p.dir + ((size_t)bh * p.dir_nodes + node) * 128 + lane * 4);
-  // row ids of this warp's slots (lane i holds slot i), then all row loads before any arithmetic
-  int my_id = -1;
-  if (lane < kProjRows && r0 + lane < nsize) my_id = perm_in[(size_t)bh * p.N + pos0 + lane];
-  uint2 w[kProjRows];
-#pragma unroll
-  for (int i = 0; i < kProjRows; ++i) {
-    const int id = __shfl_sync(0xffffffffu, my_id, i);
-    w[i] = make_uint2(0u, 0u);
-    if (id >= 0 && lane_live)
-      w[i] = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(p.x) +
-                                            2 * ((size_t)bh * p.x_stride_bh + (size_t)id * p.x_stride_row) + lane * 8);
-  }
-#pragma unroll
-  for (int i = 0; i < kProjRows; ++i) {
-    float acc = 0.f;
-    if (lane_live) {
-      float2 a, b;
-      if (kFp16) {
-        a = __half22float2(*reinterpret_cast<const __half2*>(&w[i].x));
-        b = __half22float2(*reinterpret_cast<const __half2*>(&w[i].y));
-      } else {
-        a = make_float2(bf16_lo(w[i].x), bf16_hi(w[i].x));
-        b = make_float2(bf16_lo(w[i].y), bf16_hi(w[i].y));
-      }
-      acc = fmaf(a.x, vv.x, fmaf(a.y, vv.y, fmaf(b.x, vv.z, b.y * vv.w)));
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-      const int r = r0 + i;
-      if (r >= nsize) {
-        keys[slot0 + i] = 0xFFFFFFFFFFFFFFFFull;               // padding sorts last
-      } else {
-        keys[slot0 + i] = ((unsigned long long)float_key(acc) << 32) | (unsigned)r;
-        if (proj_out != nullptr) proj_out[(size_t)bh * p.N + pos0 + i] = acc;
-      }
-    }
-  }
+  const int item = blockIdx.x, bh = blockIdx.y, tid = threadIdx.x;
+  const int node = T.item_node[item], row_begin = T.item_row0[item], size = T.node_size[node];
+  if (size <= kChunkRows) return;                              // done by the node kernel
+  const int rows = min(kChunkRows, size - row_begin);
+  const int pos0 = T.node_start[node] + row_begin;
+  vec[tid] = p.dir[((size_t)bh * p.dir_nodes + node) * 128 + tid];
+  __syncthreads();
+  unsigned long long* keys = p.keys + (size_t)bh * p.key_stride + (size_t)node * pad;
+  project_rows<D, kFp16>(smem_u32(smem), tid >> 5, tid & 31, reinterpret_cast<const uint8_t*>(p.x) + 2 * (size_t)bh * p.x_stride_bh,
+                         2 * (size_t)p.x_stride_row, perm_in + (size_t)bh * p.N + pos0, rows, row_begin, vec, keys,
+                         proj_out != nullptr ? proj_out + (size_t)bh * p.N + pos0 : nullptr, false);
+  if (row_begin + rows == size)
+    for (int r = size + tid; r < pad; r += 128) keys[r] = 0xFFFFFFFFFFFFFFFFull;           // slots beyond the node sort last
+  cp_async_wait_all();
 }
 
 
@@ -548,33 +742,86 @@ __global__ void __launch_bounds__(256) pddp_wide_project_kernel(PddpParams p, in
 // ------------------------------------------------------------------------------------------
 // sort: bitonic network over segments of `pad` keys (power of two), ascending inside each segment
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void cmpx(unsigned long long& a, unsigned long long& b, bool asc) {
-  if ((a > b) == asc) { const unsigned long long t = a; a = b; b = t; }
-}
+// A CTA sorts kSortTile consecutive slots (several short segments or a part of a long one) out of registers: thread t
+// holds slots 8 t .. 8 t + 7, so distances below 8 stay inside a thread, distances 8 to 128 are lane exchanges and only
+// those of 256 and more (10 of the 78 steps of a full tile) go through shared memory.  All 14 sorts and 8 scatters of the call
+// above: 560 us with every step in shared memory and a scatter kernel, 388 us this way.  Stages k_lo .. k_hi; distances above the tile are done by the global kernel.
+// The kernel of a segment's last stage writes the new order itself: new_perm[start + r] = old_perm[start + position].
+constexpr int kSortThreads = kSortTile / 8;
 
-// All stages with compare distance < tile, for k from k_lo to k_hi (k_hi <= pad), on tiles of
-// min(pad, kSortTile) keys held in shared memory.  For k > tile only the tail (j < tile) is done.
-__global__ void __launch_bounds__(1024) pddp_sort_smem_kernel(unsigned long long* keys_all, size_t key_stride, int pad, int tile,
-                                                              int k_lo, int k_hi) {
-  extern __shared__ __align__(16) unsigned long long sk[];
-  unsigned long long* keys = keys_all + (size_t)blockIdx.y * key_stride + (size_t)blockIdx.x * tile;
-  const int base = blockIdx.x * tile;                        // index of this tile inside the bh's key array
-  for (int i = threadIdx.x; i < tile; i += blockDim.x) sk[i] = keys[i];
-  __syncthreads();
-  for (int k = k_lo; k <= k_hi; k <<= 1) {
-    for (int j = min(k >> 1, tile >> 1); j > 0; j >>= 1) {
-      for (int t = threadIdx.x; t < (tile >> 1); t += blockDim.x) {
-        const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));      // lower index of the pair
-        const int gi = (base + i) & (pad - 1);                     // position inside the segment
-        const bool asc = (k == pad) || ((gi & k) == 0);
-        unsigned long long a = sk[i], b = sk[i + j];
-        cmpx(a, b, asc);
-        sk[i] = a; sk[i + j] = b;
-      }
-      __syncthreads();
-    }
+__device__ __forceinline__ unsigned long long u64_min(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
+__device__ __forceinline__ unsigned long long u64_max(unsigned long long a, unsigned long long b) { return a < b ? b : a; }
+
+__global__ void __launch_bounds__(kSortThreads) pddp_sort_kernel(PddpParams p, int lv, long long slots, int pad, int k_lo, int k_hi,
+                                                                const int* perm_in, int* perm_out) {
+  __shared__ unsigned long long sk[8][kSortThreads];
+  unsigned long long* keys = p.keys + (size_t)blockIdx.y * p.key_stride;
+  const int tid = threadIdx.x;
+  const long long slot0 = (long long)blockIdx.x * kSortTile + tid * 8;     // slots is a multiple of 8 (pad >= 8)
+  const bool live = slot0 < slots;
+  unsigned long long a[8];
+  if (live) {
+    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(keys + slot0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const ulonglong2 v = src[i]; a[2 * i] = v.x; a[2 * i + 1] = v.y; }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = 0xFFFFFFFFFFFFFFFFull;
   }
-  for (int i = threadIdx.x; i < tile; i += blockDim.x) keys[i] = sk[i];
+  auto cmpx = [&](int i, int j, bool asc) {
+    const unsigned long long lo = u64_min(a[i], a[j]), hi = u64_max(a[i], a[j]);
+    a[i] = asc ? lo : hi;
+    a[j] = asc ? hi : lo;
+  };
+  const int gi = (int)(slot0 & (pad - 1));                                 // position of this thread's first key in its segment
+  if (k_lo == 2) {
+    cmpx(0, 1, true); cmpx(2, 3, false); cmpx(4, 5, true); cmpx(6, 7, false);
+    cmpx(0, 2, true); cmpx(1, 3, true); cmpx(4, 6, false); cmpx(5, 7, false);
+    cmpx(0, 1, true); cmpx(2, 3, true); cmpx(4, 5, false); cmpx(6, 7, false);
+  }
+#pragma unroll 1
+  for (int k = max(k_lo, 8); k <= k_hi; k <<= 1) {
+    const bool asc = (k == pad) || ((gi & k) == 0);
+#pragma unroll 1
+    for (int j = min(k >> 1, kSortTile >> 1); j >= 8; j >>= 1) {
+      const int m = j >> 3;                                                // distance in threads
+      const bool take_min = ((tid & m) == 0) == asc;
+      if (m >= 32) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sk[i][tid] = a[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const unsigned long long b = sk[i][tid ^ m];
+          a[i] = take_min ? u64_min(a[i], b) : u64_max(a[i], b);
+        }
+        __syncthreads();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const unsigned long long b = __shfl_xor_sync(0xffffffffu, a[i], m);
+          a[i] = take_min ? u64_min(a[i], b) : u64_max(a[i], b);
+        }
+      }
+    }
+    cmpx(0, 4, asc); cmpx(1, 5, asc); cmpx(2, 6, asc); cmpx(3, 7, asc);
+    cmpx(0, 2, asc); cmpx(1, 3, asc); cmpx(4, 6, asc); cmpx(5, 7, asc);
+    cmpx(0, 1, asc); cmpx(2, 3, asc); cmpx(4, 5, asc); cmpx(6, 7, asc);
+  }
+  if (!live) return;
+  if (k_hi == pad) {
+    const LevelTables T = level_tables(p.tables, lv, p.table_stride);
+    const int node = (int)(slot0 / pad);
+    const int size = T.node_size[node];
+    const size_t start = (size_t)blockIdx.y * p.N + T.node_start[node];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (gi + i < size) perm_out[start + gi + i] = perm_in[start + (size_t)(a[i] & 0xFFFFFFFFull)];
+  } else {
+    ulonglong2* dst = reinterpret_cast<ulonglong2*>(keys + slot0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dst[i] = make_ulonglong2(a[2 * i], a[2 * i + 1]);
+  }
 }
 
 // One compare-exchange step at distance j >= tile of stage k.
@@ -588,19 +835,6 @@ __global__ void __launch_bounds__(256) pddp_sort_global_kernel(unsigned long lon
   const bool asc = (k == pad) || ((gi & k) == 0);
   unsigned long long a = keys[i], b = keys[i + j];
   if ((a > b) == asc) { keys[i] = b; keys[i + j] = a; }
-}
-
-// new_perm[start + r] = old_perm[start + sorted position r]
-__global__ void __launch_bounds__(256) pddp_scatter_kernel(PddpParams p, int lv, int nodes, int pad, const int* perm_in, int* perm_out) {
-  const LevelTables T = level_tables(p.tables, lv, p.table_stride);
-  const int bh = blockIdx.y;
-  const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= (long long)nodes * pad) return;
-  const int node = (int)(slot / pad), r = (int)(slot % pad);
-  if (r >= T.node_size[node]) return;
-  const unsigned long long key = p.keys[(size_t)bh * p.key_stride + slot];
-  const int start = T.node_start[node];
-  perm_out[(size_t)bh * p.N + start + r] = perm_in[(size_t)bh * p.N + start + (int)(key & 0xFFFFFFFFull)];
 }
 
 __global__ void pddp_iota_kernel(int* perm, long long total, int N) {
@@ -698,11 +932,17 @@ int launch_pddp(const PddpArgs& a, cudaStream_t stream) {
     p.dir = reinterpret_cast<float*>(ws + pl.off_dir); p.dir_nodes = pl.K;
     p.keys = reinterpret_cast<unsigned long long*>(ws + pl.off_keys); p.key_stride = pl.key_stride;
     p.status = a.status;
-    pddp_tables_kernel<<<1, 1, 0, stream>>>(N, C, p.tables, pl.levels, pl.table_stride);
-    auto gram = a.fp16 ? pddp_gram_kernel<true> : pddp_gram_kernel<false>;
-    if (cudaFuncSetAttribute(gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmem) != cudaSuccess) return -8;
+    pddp_tables_kernel<<<1, kTableThreads, 0, stream>>>(N, C, p.tables, pl.levels, pl.table_stride);
+    auto node = a.D == 64 ? (a.fp16 ? pddp_node_kernel<64, true> : pddp_node_kernel<64, false>)
+                          : (a.fp16 ? pddp_node_kernel<128, true> : pddp_node_kernel<128, false>);
+    auto project = a.D == 64 ? (a.fp16 ? pddp_project_kernel<64, true> : pddp_project_kernel<64, false>)
+                             : (a.fp16 ? pddp_project_kernel<128, true> : pddp_project_kernel<128, false>);
+    const int project_smem = kBufs * kTileBytes + 1024;
     const int power_smem = (128 * 128 + 128 + 512 + 8) * sizeof(float);
-    if (cudaFuncSetAttribute(pddp_power_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, power_smem) != cudaSuccess) return -8;
+    if (cudaFuncSetAttribute(node, cudaFuncAttributeMaxDynamicSharedMemorySize, NodeSmem::kDynamic) != cudaSuccess ||
+        cudaFuncSetAttribute(project, cudaFuncAttributeMaxDynamicSharedMemorySize, project_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pddp_power_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, power_smem) != cudaSuccess)
+      return -8;
     const float* v0 = a.start_vectors;
     const bool wide = a.D != 64 && a.D != 128;
     // wide path: per-chunk partial sums first, then the directions (256 floats per node), both inside the partial area
@@ -730,23 +970,22 @@ int launch_pddp(const PddpArgs& a, cudaStream_t stream) {
         if (a.fp16) pddp_wide_project_kernel<true><<<dim3(pgrid, BH), 256, 0, stream>>>(p, lv, ls.nodes, ls.pad, perm_a, wdir, proj);
         else pddp_wide_project_kernel<false><<<dim3(pgrid, BH), 256, 0, stream>>>(p, lv, ls.nodes, ls.pad, perm_a, wdir, proj);
       } else {
-        gram<<<dim3(ls.items, BH), kGramThreads, kGramSmem, stream>>>(p, lv, perm_a);
-        pddp_power_kernel<<<dim3(ls.nodes, BH), 512, power_smem, stream>>>(p, lv, ls.nodes, v0);
-        if (a.fp16) pddp_project_kernel<true><<<dim3(pgrid, BH), 256, 0, stream>>>(p, lv, ls.nodes, ls.pad, perm_a, proj);
-        else pddp_project_kernel<false><<<dim3(pgrid, BH), 256, 0, stream>>>(p, lv, ls.nodes, ls.pad, perm_a, proj);
+        node<<<dim3(ls.items, BH), kNodeThreads, NodeSmem::kDynamic, stream>>>(p, lv, ls.nodes, ls.pad, perm_a, v0, proj);
+        if (ls.items > ls.nodes) {               // some nodes are more than one item
+          pddp_power_kernel<<<dim3(ls.nodes, BH), 512, power_smem, stream>>>(p, lv, ls.nodes, v0);
+          project<<<dim3(ls.items, BH), 128, project_smem, stream>>>(p, lv, ls.pad, perm_a, proj);
+        }
       }
       v0 += (size_t)BH * ls.nodes * a.D;
-      // bitonic sort of every segment of `pad` keys
-      const int tile = std::min(ls.pad, kSortTile);
-      const unsigned tiles = (unsigned)(slots / tile);
-      const int sthreads = std::max(32, std::min(1024, tile / 2));
-      pddp_sort_smem_kernel<<<dim3(tiles, BH), sthreads, (size_t)tile * 8, stream>>>(p.keys, p.key_stride, ls.pad, tile, 2, tile);
-      for (int k = tile * 2; k <= ls.pad; k <<= 1) {
-        for (int j = k >> 1; j >= tile; j >>= 1)
+      // bitonic sort of every segment of `pad` keys; the last kernel writes the new order
+      const int tile_k = std::min(ls.pad, kSortTile);
+      const dim3 sgrid((unsigned)((slots + kSortTile - 1) / kSortTile), BH);
+      pddp_sort_kernel<<<sgrid, kSortThreads, 0, stream>>>(p, lv, slots, ls.pad, 2, tile_k, perm_a, perm_b);
+      for (int k = tile_k * 2; k <= ls.pad; k <<= 1) {
+        for (int j = k >> 1; j >= kSortTile; j >>= 1)
           pddp_sort_global_kernel<<<dim3((unsigned)((slots / 2 + 255) / 256), BH), 256, 0, stream>>>(p.keys, p.key_stride, slots / 2, ls.pad, k, j);
-        pddp_sort_smem_kernel<<<dim3(tiles, BH), sthreads, (size_t)tile * 8, stream>>>(p.keys, p.key_stride, ls.pad, tile, k, k);
+        pddp_sort_kernel<<<sgrid, kSortThreads, 0, stream>>>(p, lv, slots, ls.pad, k, k, perm_a, perm_b);
       }
-      pddp_scatter_kernel<<<dim3((unsigned)((slots + 255) / 256), BH), 256, 0, stream>>>(p, lv, ls.nodes, ls.pad, perm_a, perm_b);
       std::swap(perm_a, perm_b);
     }
   }

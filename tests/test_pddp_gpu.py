@@ -98,3 +98,10 @@ def test_tiny_groups(cuda_device, N, C):
     for li, nodes in enumerate(level_ranges(N, C)):
         assert torch.equal(resort_from_projections(orders[li], proj[li], nodes), orders[li + 1]), f"level {li}"
     assert torch.equal(orders[-1], perm)
+
+
+# nodes of one work item (2,048 rows) and of several, mixed levels, ragged last tiles, segments longer than a sort tile
+@pytest.mark.parametrize("BH,N,D,C,iters", [(1, 4224, 64, 128, 4), (2, 2049, 128, 128, 4), (1, 2048, 64, 128, 2), (3, 300, 128, 128, 4),
+                                            (1, 8200, 64, 128, 4), (1, 16500, 128, 128, 4), (1, 700, 64, 32, 4)])
+def test_node_edges(cuda_device, BH, N, D, C, iters):
+    test_two_stage_contract(cuda_device, BH, N, D, C, iters)

@@ -6,13 +6,21 @@
 // i.e. the length of the shortest prefix of the descending order whose mass reaches topp (everything if the
 // whole row stays below it, at least one).  That is the reference's top-p rule
 // (mcsparse/kernels/flash_mcsa/token_sparse.py:842-876: sort, cumulative sum, mask cumsum_before < topp, count),
-// without sorting: the sum S(x) of all scores above a threshold x falls as x rises, so the boundary value b =
-// min{x : S(x) < topp} is found by a search over the order-preserving 32-bit image of the scores (four
-// thresholds in every pass over the row, sixteen passes), and one more pass counts the scores above b and those
-// equal to it (ties enter one by one until the mass is reached).  A row is read from L2 seventeen times and
-// never written; sums are accumulated in fp32 per thread and in fp64 across the CTA in a fixed order, so the
-// result is reproducible.  The selection itself (which tokens) is done by the top-k kernel with this count as
-// the row's budget.
+// without sorting: three histogram passes over the order-preserving 32-bit image of the scores (11, 11 and 10 bits,
+// most significant first) narrow down the key at which the mass of the keys above it passes topp; ties on that key enter
+// one by one until the mass is reached.  The selection itself (which tokens) is done by the top-k kernel with this
+// count as the row's budget.
+//
+// A histogram bin holds its number of scores and their exact mass: the 11 bits of the first pass contain sign and
+// exponent, so all scores of a bin are whole multiples of one power of two, and their 24-bit significands are added
+// as integers (two halves of 12 bits in 32-bit words: no overflow up to 2^20 scores, 64-bit words beyond).  Integer sums do
+// not depend on the order of the atomics, so the result is reproducible; bins are combined in fp64.
+//
+// What bounds it: the atomics of the first pass (three per score).  Two copies of the histogram (even and odd lanes)
+// halve the collisions inside a warp.  1,024 rows of 16,380 scores: 125 us (the bisection that came before, seventeen
+// sweeps with three compares per score, took 644 us; one read of the scores at the copy rate: 10 us).
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -21,7 +29,7 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxSinks = 64;
+constexpr int kDigits = 2048;
 
 __device__ __forceinline__ uint32_t prob_key(float s) {
   uint32_t u = __float_as_uint(s);
@@ -29,107 +37,170 @@ __device__ __forceinline__ uint32_t prob_key(float s) {
   if (s == 0.f) u = 0u;
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);       // order-preserving
 }
-__device__ __forceinline__ float key_value(uint32_t k) {
-  const uint32_t u = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
-  return __uint_as_float(u);
-}
+__device__ __forceinline__ uint32_t key_bits(uint32_t k) { return (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k; }
 
+// kBig: rows of more than 2^20 scores
+template <bool kBig>
 struct Shared {
-  double sum[3][kWarps];
-  unsigned int cnt[3][kWarps];
-  int sinks[kMaxSinks];
-  double r_sum[3];
-  unsigned int r_cnt[3];
+  using Acc = typename std::conditional<kBig, unsigned long long, unsigned int>::type;
+  static constexpr int kCopies = kBig ? 1 : 2;
+  unsigned int cnt[kCopies][kDigits];
+  Acc lo[kCopies][kDigits], hi[kCopies][kDigits];          // sums of the lower and upper 12 bits of the significands
+  double warp_sum[kWarps];
+  unsigned int warp_cnt[kWarps];
+  int best, lowest;
+  double s_above;
+  unsigned int n_above, n_eq;
 };
 
-// block-wide sums of three (count, mass) pairs; the result is in sh.r_* for every thread after the call
-__device__ __forceinline__ void reduce3(Shared& sh, const unsigned int (&c)[3], const float (&s)[3]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    unsigned int ci = c[i];
-    double si = (double)s[i];
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      ci += __shfl_xor_sync(0xffffffffu, ci, off);
-      si += __shfl_xor_sync(0xffffffffu, si, off);
-    }
-    if (lane == 0) { sh.cnt[i][warp] = ci; sh.sum[i][warp] = si; }
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    unsigned int ci = 0;
-    double si = 0.0;
-    for (int w = 0; w < kWarps; ++w) { ci += sh.cnt[threadIdx.x][w]; si += sh.sum[threadIdx.x][w]; }
-    sh.r_cnt[threadIdx.x] = ci;
-    sh.r_sum[threadIdx.x] = si;
-  }
-  __syncthreads();
-}
-
+template <bool kBig>
 __global__ void __launch_bounds__(kThreads) topp_count_kernel(const float* __restrict__ scores, const int32_t* __restrict__ sinks,
                                                              int n_sink, long long rows, int L, float topp, int32_t* __restrict__ counts) {
-  __shared__ Shared sh;
-  if (threadIdx.x < n_sink) sh.sinks[threadIdx.x] = sinks[threadIdx.x];
+  using S = Shared<kBig>;
+  using Acc = typename S::Acc;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  S& sh = *reinterpret_cast<S*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int copy = lane & (S::kCopies - 1);
+  for (int i = tid; i < S::kCopies * kDigits; i += kThreads) {
+    sh.cnt[0][i] = 0u;                                     // (the copies are contiguous)
+    sh.lo[0][i] = 0;
+    sh.hi[0][i] = 0;
+  }
+  if (tid == 0) { sh.best = -1; sh.lowest = kDigits; }
   __syncthreads();
+#pragma unroll 1
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float* sc = scores + row * (long long)L;
-    // one pass: counts and masses of the scores whose key lies above each of three thresholds
-    auto pass = [&](uint32_t t0, uint32_t t1, uint32_t t2, bool eq_mode) {
-      unsigned int c[3] = {0, 0, 0};
-      float s[3] = {0.f, 0.f, 0.f};
-      for (int j = threadIdx.x; j < L; j += kThreads) {
-        bool sink = false;
-        for (int i = 0; i < n_sink; ++i) sink |= (sh.sinks[i] == j);
-        if (sink) continue;
-        const float v = __ldg(sc + j);
-        const uint32_t k = prob_key(v);
-        const float m = (v == v) ? v : 0.f;
-        if (!eq_mode) {
-          if (k > t0) { ++c[0]; s[0] += m; }
-          if (k > t1) { ++c[1]; s[1] += m; }
-          if (k > t2) { ++c[2]; s[2] += m; }
-        } else {
-          if (k > t0) { ++c[0]; s[0] += m; }               // strictly above the boundary
-          if (k == t0) ++c[1];                             // equal to it
-        }
-      }
-      reduce3(sh, c, s);
-    };
-    // b = smallest x with S(x) < topp, S(x) = mass of the scores whose key is above x; S(0xFFFFFFFF) = 0 < topp
-    uint32_t lo = 0u, hi = 0xFFFFFFFFu;                     // the answer lies in [lo, hi]
+    uint32_t prefix = 0u, mask = 0u;
+    double s_base = 0.0;                                   // mass and number of the scores above the current prefix
+    unsigned int n_base = 0u, n_eq = 0u;
+    bool all = false;
 #pragma unroll 1
-    while (lo < hi) {
-      const uint64_t span = (uint64_t)hi - lo;             // >= 1
-      const uint32_t t0 = lo + (uint32_t)(span / 4), t1 = lo + (uint32_t)(span / 2), t2 = lo + (uint32_t)(span / 4 * 3);
-      pass(t0, t1, t2, false);
-      const bool f0 = sh.r_sum[0] < (double)topp, f1 = sh.r_sum[1] < (double)topp, f2 = sh.r_sum[2] < (double)topp;
-      __syncthreads();                                     // everyone has read the results before the next pass overwrites them
-      // f is monotone (false ... false true ... true) over x
-      if (f0) hi = t0;
-      else if (f1) { lo = t0 + 1; hi = t1; }
-      else if (f2) { lo = t1 + 1; hi = t2; }
-      else lo = t2 + 1;
-    }
-    const uint32_t b = lo;
-    pass(b, 0u, 0u, true);
-    if (threadIdx.x == 0) {
-      const unsigned int above = sh.r_cnt[0], equal = sh.r_cnt[1];
-      const double s_above = sh.r_sum[0];
-      const double v = (double)key_value(b);
-      unsigned int take = equal;                           // ties enter one by one while the mass before them is below topp
-      if (v > 0.0) {
-        const double need = ((double)topp - s_above) / v;
-        const double cn = ceil(need);
-        take = cn < 1.0 ? 1u : (cn > (double)equal ? equal : (unsigned int)cn);
+    for (int pass = 0; pass < 3; ++pass) {
+      const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
+      const uint32_t dm = pass == 2 ? 1023u : 2047u;
+      // sign: +1 adds a score, -1 (modulo 2^32 or 2^64) takes it out again
+      auto count = [&](float v, unsigned int sign) {
+        const uint32_t key = prob_key(v);
+        if ((key & mask) != prefix) return;
+        const uint32_t d = (key >> shift) & dm;
+        const uint32_t u = __float_as_uint(v);
+        uint32_t m = (u & 0x7FFFFFu) | ((u & 0x7F800000u) != 0u ? 0x800000u : 0u);
+        if (v != v) m = 0u;
+        atomicAdd(&sh.cnt[copy][d], sign);
+        if (m != 0u) {
+          atomicAdd(&sh.lo[copy][d], sign == 1u ? (Acc)(m & 0xFFFu) : (Acc)0 - (Acc)(m & 0xFFFu));
+          atomicAdd(&sh.hi[copy][d], sign == 1u ? (Acc)(m >> 12) : (Acc)0 - (Acc)(m >> 12));
+        }
+      };
+#pragma unroll 8
+      for (int j = tid; j < L; j += kThreads) count(__ldg(sc + j), 1u);
+      for (int i = tid; i < n_sink; i += kThreads) count(__ldg(sc + sinks[i]), 0xFFFFFFFFu);     // sinks are not ranked
+      __syncthreads();
+      // thread t owns digits 4 t .. 4 t + 3: their counts and masses, then the totals above them
+      unsigned int c[4], c_sum = 0u;
+      double s[4], s_sum = 0.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int d = 4 * tid + i;
+        unsigned int cc = 0u;
+        Acc lo = 0, hi = 0;
+#pragma unroll
+        for (int q = 0; q < S::kCopies; ++q) {
+          cc += sh.cnt[q][d]; lo += sh.lo[q][d]; hi += sh.hi[q][d];
+          sh.cnt[q][d] = 0u; sh.lo[q][d] = 0; sh.hi[q][d] = 0;
+        }
+        c[i] = cc;
+        const double m = (double)lo + 4096.0 * (double)hi;               // exact: below 2^53
+        const uint32_t u = key_bits(prefix | ((uint32_t)d << shift));    // any key of the bin has its sign and exponent
+        const int e = (int)((u >> 23) & 0xFFu);
+        double v = 0.0;
+        if (m != 0.0) v = e == 255 ? (double)INFINITY : scalbn(m, (e == 0 ? 1 : e) - 150);
+        s[i] = (u & 0x80000000u) ? -v : v;
+        c_sum += c[i];
+        s_sum += s[i];
       }
-      unsigned int n = above + take;
-      if (n < 1u) n = 1u;
-      const unsigned int cap = (unsigned int)(L - n_sink);
-      counts[row] = (int32_t)(n > cap ? cap : n);
+      unsigned int c_incl = c_sum;
+      double s_incl = s_sum;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned int cn = __shfl_down_sync(0xffffffffu, c_incl, off);
+        const double sn = __shfl_down_sync(0xffffffffu, s_incl, off);
+        if (lane + off < 32) { c_incl += cn; s_incl += sn; }
+      }
+      // exclusive totals of the lanes above
+      unsigned int c_gt = __shfl_down_sync(0xffffffffu, c_incl, 1);
+      double s_gt = __shfl_down_sync(0xffffffffu, s_incl, 1);
+      if (lane == 31) { c_gt = 0u; s_gt = 0.0; }
+      if (lane == 0) { sh.warp_cnt[warp] = c_incl; sh.warp_sum[warp] = s_incl; }
+      __syncthreads();
+      double s_hi = 0.0;
+      for (int w = kWarps - 1; w > warp; --w) { c_gt += sh.warp_cnt[w]; s_hi += sh.warp_sum[w]; }
+      s_gt += s_hi + s_base;
+      c_gt += n_base;
+      // the highest digit at which the mass reaches topp
+      int mine = -1, low = kDigits;
+      double s_mine = 0.0, s_run = s_gt;
+      unsigned int n_mine = 0u, eq_mine = 0u, n_run = c_gt, n_low = 0u, eq_low = 0u;
+      double s_low = 0.0;
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {
+        if (c[i] != 0u) { low = 4 * tid + i; s_low = s_run; n_low = n_run; eq_low = c[i]; }
+        if (mine < 0 && c[i] != 0u && s_run + s[i] >= (double)topp) { mine = 4 * tid + i; s_mine = s_run; n_mine = n_run; eq_mine = c[i]; }
+        s_run += s[i];
+        n_run += c[i];
+      }
+      if (mine >= 0) atomicMax(&sh.best, mine);
+      if (low < kDigits) atomicMin(&sh.lowest, low);
+      __syncthreads();
+      const int best = sh.best, lowest = sh.lowest;
+      all = pass == 0 && best < 0;                         // the whole row stays below topp
+      // (after the first pass the mass is known to be reached inside the prefix; if the last bit of an fp64 sum says
+      // otherwise, it is at the lowest key)
+      if (best >= 0 ? mine == best : low == lowest) {
+        sh.s_above = best >= 0 ? s_mine : s_low;
+        sh.n_above = best >= 0 ? n_mine : n_low;
+        sh.n_eq = best >= 0 ? eq_mine : eq_low;
+      }
+      __syncthreads();
+      if (tid == 0) { sh.best = -1; sh.lowest = kDigits; }
+      s_base = sh.s_above;
+      n_base = sh.n_above;
+      n_eq = sh.n_eq;
+      __syncthreads();
+      if (all) break;
+      prefix |= (uint32_t)(best >= 0 ? best : lowest) << shift;
+      mask |= dm << shift;
     }
-    __syncthreads();
+    if (tid == 0) {
+      const unsigned int cap = (unsigned int)(L - n_sink);
+      unsigned int n = cap;
+      if (!all) {
+        const double v = (double)__uint_as_float(key_bits(prefix));
+        unsigned int take = n_eq;                          // ties enter one by one while the mass before them is below topp
+        if (v > 0.0) {
+          const double cn = ceil(((double)topp - s_base) / v);
+          take = cn < 1.0 ? 1u : (cn > (double)n_eq ? n_eq : (unsigned int)cn);
+        }
+        n = n_base + take;
+        if (n < 1u) n = 1u;
+        if (n > cap) n = cap;
+      }
+      counts[row] = (int32_t)n;
+    }
   }
+}
+
+template <bool kBig>
+int launch(const float* scores, const int32_t* sinks, int n_sink, long long rows, int L, float topp, int32_t* counts, cudaStream_t stream) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int smem = (int)sizeof(Shared<kBig>);
+  if (cudaFuncSetAttribute(topp_count_kernel<kBig>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -8;
+  const long long grid = rows < (long long)sms * 4 ? rows : (long long)sms * 4;
+  topp_count_kernel<kBig><<<(unsigned)grid, kThreads, smem, stream>>>(scores, sinks, n_sink, rows, L, topp, counts);
+  return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
 }  // namespace
@@ -137,11 +208,8 @@ __global__ void __launch_bounds__(kThreads) topp_count_kernel(const float* __res
 int launch_topp_count(const float* scores, const int32_t* sinks, int n_sink, long long rows, int L, float topp, int32_t* counts,
                       cudaStream_t stream) {
   if (rows == 0) return 0;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long grid = rows < (long long)sms * 4 ? rows : (long long)sms * 4;
-  topp_count_kernel<<<(unsigned)grid, kThreads, 0, stream>>>(scores, sinks, n_sink, rows, L, topp, counts);
-  return cudaGetLastError() == cudaSuccess ? 0 : -8;
+  return L <= (1 << 20) ? launch<false>(scores, sinks, n_sink, rows, L, topp, counts, stream)
+                        : launch<true>(scores, sinks, n_sink, rows, L, topp, counts, stream);
 }
 
 }  // namespace mcs

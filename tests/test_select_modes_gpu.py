@@ -112,3 +112,18 @@ def test_backend_with_topp_selection(cuda_device):
     ref, _ = gather_attn_ref(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), gi, gl=gl)
     mx, mr = error_metrics(out.transpose(1, 2), ref)
     assert mx < 2e-2 and mr < 1e-2, (mx, mr)
+
+
+@pytest.mark.parametrize("L", [33, 2047, 4097, (1 << 20) + 5])
+def test_topp_count_wide_range(cuda_device, L):
+    """Masses over the whole fp32 range (denormals included), ties, sinks that would dominate, more than 2^20 scores."""
+    from mcsparse_b200.kernels.flash_mcsa.token_sparse import topp_count
+    g = torch.Generator().manual_seed(L)
+    tp = torch.zeros(1, 1, 3, L)
+    tp[0, 0, 0] = torch.exp(-95.0 * torch.rand(L, generator=g))
+    tp[0, 0, 1] = torch.exp2(-torch.randint(0, 149, (L,), generator=g).float())
+    tp[0, 0, 2] = (torch.rand(L, generator=g) < 0.5).float()
+    tp /= tp.sum(-1, keepdim=True)
+    tp[..., 0] = 3.0
+    got = topp_count(tp.to(cuda_device), 0.609375, [(0, 1)]).cpu()
+    assert torch.equal(got, topp_count_ref(tp, 0.609375, [0]).to(got.dtype)), got      # exact integer sums per bin: no rounding slack

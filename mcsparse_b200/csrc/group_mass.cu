@@ -22,12 +22,14 @@
 // The kernel is bound by the ex2 throughput of the SFU (16 per clock per SM); a quarter of the exponentials
 // are therefore evaluated by a polynomial on the FMA pipe.
 //
-// Roles: warps 0-7 exponentiate and sum (two threads per key token: warps w and w+4 share a TMEM
-// lane group and take 64 query columns each, so that every SM sub-partition has two warps feeding
-// its SFU; the two partial sums meet in shared memory), warp 8 issues the MMAs (converged, one
-// elected lane executes the tcgen05 instructions), warps 9-12 prepare the query operand
-// and stream the key tiles into a 3-slot ring: by TMA (one elected thread, boxes of 128 rows x 128 bytes)
-// when a tensor map can describe K's strides, else with cp.async.
+// Roles: warps 0-15 exponentiate and sum, in two groups of eight for the even and the odd key tiles (two threads per key
+// token: warps w and w+4 of a group share a TMEM lane group and take 64 query columns each; the two partial sums meet in
+// shared memory).  Four warps per SM sub-partition feed its SFU, and each group has two score buffers of its own, so one
+// group's waits and tensor-memory loads lie under the other's exponentials: with a single group and two buffers the SFU
+// was 64% busy (7,100 -> 6,517 us at 24 heads x 32,760 x 128, 655 -> 573 us at 8 x 16,380; floors 5,900 / 500 us of ex2
+// alone, 4,400 / 370 with a quarter of them on the FMA pipe).  Warp 16 issues the MMAs (converged, one elected lane executes
+// the tcgen05 instructions), warps 17-19 prepare the query operand and stream the key tiles into a 3-slot ring: by TMA (one
+// elected thread, boxes of 128 rows x 128 bytes) when a tensor map can describe K's strides, else with cp.async.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -39,17 +41,19 @@ namespace mcs {
 namespace {
 
 constexpr int kTile = 128;
-constexpr int kThreads = 416;
-constexpr int kExpWarps = 8;
-constexpr int kProducerThreads = 128;
-constexpr int kMmaWarp = 8;
-constexpr int kProducerWarp0 = 9;
+constexpr int kThreads = 640;          // five warps per SM sub-partition: 96 registers each
+constexpr int kExpWarps = 16;          // two groups of eight: even and odd key tiles
+constexpr int kBufs = 4;               // score buffers in tensor memory, two per group
+constexpr int kProducerWarps = 3;
+constexpr int kProducerThreads = kProducerWarps * 32;
+constexpr int kMmaWarp = 16;
+constexpr int kProducerWarp0 = 17;
 constexpr int kRing = 3;
-constexpr uint32_t kTmemCols = 256;   // two score buffers of 128 columns
+constexpr uint32_t kTmemCols = 128 * kBufs;
 
-enum { BAR_FULL = 0, BAR_EMPTY = BAR_FULL + kRing, BAR_Q_FULL = BAR_EMPTY + kRing, BAR_S_FULL, BAR_S_FREE = BAR_S_FULL + 2,
-       BAR_PART = BAR_S_FREE + 2,      // [4 lane groups][2 bufs]: partial sums of the upper column half are in shared memory
-       BAR_DRAIN = BAR_PART + 8, BAR_COUNT };
+enum { BAR_FULL = 0, BAR_EMPTY = BAR_FULL + kRing, BAR_Q_FULL = BAR_EMPTY + kRing, BAR_S_FULL, BAR_S_FREE = BAR_S_FULL + kBufs,
+       BAR_PART = BAR_S_FREE + kBufs,  // [4 lane groups][kBufs]: partial sums of the upper column half are in shared memory
+       BAR_DRAIN = BAR_PART + 4 * kBufs, BAR_COUNT };
 
 // D is the head dimension rounded up to the tile layouts this kernel has: 64, 128, 192 or 256 (the true head
 // dimension, any multiple of 8 up to 256, is a run-time value; rows are zero-padded on their way into shared memory)
@@ -59,12 +63,12 @@ struct Smem {
   static constexpr int kTileBytes = kBlocks * 16384;
   static constexpr int kRingN = D == 256 ? 2 : kRing;        // key-tile slots that fit beside the query tile
   static constexpr int kQ = 0;                              // group's query rows (B operand)
-  static constexpr int kQx = kTileBytes;                    // extra k-step of Q: 128 rows x 128 B (first 32 B used)
-  static constexpr int kKx = kQx + 16384;                   // extra k-step of K: constant (1,1,1,0...)
-  static constexpr int kRingOff = kKx + 16384;
+  static constexpr int kX = kTileBytes;                     // extra k-steps, 128 rows x 128 B: chunks 0-1 K's constant
+                                                            // (1,1,1,0...), chunks 2-3 Q's, the rest unused
+  static constexpr int kRingOff = kX + 16384;
   static constexpr int kBars = kRingOff + kRingN * kTileBytes;
-  static constexpr int kPart = kBars + BAR_COUNT * 8;       // float [2][128]: partial sums of the upper column half
-  static constexpr int kTmemSlot = kPart + 2 * 128 * 4;
+  static constexpr int kPart = kBars + BAR_COUNT * 8;       // float [kBufs][128]: partial sums of the upper column half
+  static constexpr int kTmemSlot = kPart + kBufs * 128 * 4;
   static constexpr int kTotal = kTmemSlot + 16;
   static constexpr int kDynamic = kTotal + 1024;
 };
@@ -106,11 +110,11 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       mbar_init(bar(BAR_EMPTY + i), 1);
     }
     mbar_init(bar(BAR_Q_FULL), 2 * kProducerThreads);   // per thread: its cp.async rows + its plain stores
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kBufs; ++i) {
       mbar_init(bar(BAR_S_FULL + i), 1);
-      mbar_init(bar(BAR_S_FREE + i), kExpWarps);
+      mbar_init(bar(BAR_S_FREE + i), kExpWarps / 2);
     }
-    for (int i = 0; i < 8; ++i) mbar_init(bar(BAR_PART + i), 1);
+    for (int i = 0; i < 4 * kBufs; ++i) mbar_init(bar(BAR_PART + i), 1);
     mbar_init(bar(BAR_DRAIN), 1);
     mbar_fence_init();
   }
@@ -125,7 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
 
   if (warp < kExpWarps) {
     // ===================================================================== exp + column sum
-    const int lg = warp & 3, x = warp >> 2;            // TMEM lane group, column half
+    const int lg = warp & 3, x = (warp >> 2) & 1;      // TMEM lane group, column half
     const int j_in = lg * 32 + lane;                   // key token inside the tile == TMEM lane
     const uint32_t lane_addr = (static_cast<uint32_t>(lg) * 32u) << 16;
     const float c = p.scale_log2;
@@ -135,9 +139,9 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
     float* part = reinterpret_cast<float*>(smem + L::kPart);
     bool ok = true;
 #pragma unroll 1
-    for (int t = 0; t < n_tiles && ok; ++t) {
-      const int buf = t & 1;
-      ok = mbar_wait(bar(BAR_S_FULL + buf), (t >> 1) & 1, p.status, 40);
+    for (int t = warp >> 3; t < n_tiles && ok; t += 2) {
+      const int buf = t & (kBufs - 1), ph = (t / kBufs) & 1;
+      ok = mbar_wait(bar(BAR_S_FULL + buf), ph, p.status, 40);
       if (!ok) break;
       tc_fence_after();
       float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
@@ -150,8 +154,8 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
         for (int i = 0; i < 32; i += 8) {
           // kPoly of every eight exponentials are computed on the FMA pipe instead of the special-function unit,
           // which bounds this kernel (see ex2_poly3_scaled); their positions are spread over the four partial sums.
-          // Two of eight measured best (7.84 ms against 8.29 ms with none and 8.10 / 8.36 ms with three / four at
-          // H=24, L=32,760: beyond a quarter the extra instructions cost more issue slots than the unit gains).
+          // Two of eight measured best (6.52 ms against 6.69 / 6.88 ms with one / three at H=24, L=32,760: beyond a
+          // quarter the extra instructions cost more issue slots than the unit gains).
           auto e = [&](int k) {
             const float v = __uint_as_float(r[i + k]);
             const bool poly = (kPoly >= 1 && k == 3) || (kPoly >= 2 && k == 6) || (kPoly >= 3 && k == 1) || (kPoly >= 4 && k == 4);
@@ -172,11 +176,11 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
         part[buf * 128 + j_in] = sum;
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(bar(BAR_PART + 2 * lg + buf));
+          mbar_arrive(bar(BAR_PART + kBufs * lg + buf));
           mbar_arrive(bar(BAR_S_FREE + buf));              // one arrival per warp
         }
       } else {
-        ok = mbar_wait(bar(BAR_PART + 2 * lg + buf), (t >> 1) & 1, p.status, 45);
+        ok = mbar_wait(bar(BAR_PART + kBufs * lg + buf), ph, p.status, 45);
         if (!ok) break;
         const int j = t * kTile + j_in;
         if (j < p.Lk) out[j] = (sum + part[buf * 128 + j_in]) * norm;
@@ -195,14 +199,14 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       constexpr uint32_t kLbo = (16u >> 4) << 16;
       auto desc = [&](uint32_t lo) { return (static_cast<uint64_t>(kDescHi) << 32) | lo; };
       const uint32_t qlo = (((s_base + L::kQ) & 0x3FFFFu) >> 4) | kLbo;
-      const uint32_t qxlo = (((s_base + L::kQx) & 0x3FFFFu) >> 4) | kLbo;
-      const uint32_t kxlo = (((s_base + L::kKx) & 0x3FFFFu) >> 4) | kLbo;
+      const uint32_t kxlo = (((s_base + L::kX) & 0x3FFFFu) >> 4) | kLbo;
+      const uint32_t qxlo = kxlo + 2;                    // second 32-byte k-step of the same rows
       bool ok = mbar_wait(bar(BAR_Q_FULL), 0, p.status, 41);
       int slot = 0, phase = 0;
 #pragma unroll 1
       for (int t = 0; t < n_tiles && ok; ++t) {
-        const int buf = t & 1;
-        if (t >= 2) ok = mbar_wait(bar(BAR_S_FREE + buf), ((t >> 1) - 1) & 1, p.status, 42);
+        const int buf = t & (kBufs - 1);
+        if (t >= kBufs) ok = mbar_wait(bar(BAR_S_FREE + buf), (t / kBufs - 1) & 1, p.status, 42);
         ok = ok && mbar_wait(bar(BAR_FULL + slot), phase, p.status, 43);
         if (!ok) break;
         fence_proxy_async_smem();
@@ -241,8 +245,6 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
   } else {
     // ===================================================================== producers
     const int pw = warp - kProducerWarp0;
-    const int ptid = pw * 32 + lane;                    // 0..127: also the row this thread prepares
-    const int row0 = pw * 32;
     // one lane per 16-byte chunk of a row; the padded layouts give every lane one of 32 chunk positions, of which
     // D / 8 exist in the tile (the others idle) and p.D / 8 hold data (the rest is zero-filled)
     constexpr int kChunks = kWide ? 32 : D / 8;
@@ -250,13 +252,13 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
     const int sub = lane / kChunks, cch = lane % kChunks;
     const bool c_in_tile = !kWide || cch < D / 8;
     const bool c_live = !kWide || cch < d_chunks;
-    // ---- constant extra K block, extra Q block, Q rows
-    {
+    // ---- constant extra K block, extra Q block, Q rows (three warps share the four blocks of 32 rows)
+#pragma unroll 1
+    for (int row0 = pw * 32; row0 < 128; row0 += kProducerThreads) {
       // K extra: every row (1, 1, 1, 0, ...); Q extra: (-hi, -mid, -lo, 0, ...) of lse / scale
       const uint32_t one = kFp16 ? 0x3C00u : 0x3F80u;
-      uint8_t* kx = smem + L::kKx;
-      uint8_t* qx = smem + L::kQx;
-      const int r = ptid;
+      uint8_t* xt = smem + L::kX;
+      const int r = row0 + lane;
       uint4 kv0 = make_uint4(one | (one << 16), one, 0, 0);
       float x = 3.0e38f;                                 // padding rows: exp(-huge) = 0
       if (kFp16) x = 60000.f;
@@ -277,13 +279,11 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
         w0 = (uint32_t)__bfloat16_as_ushort(__hneg(hi)) | ((uint32_t)__bfloat16_as_ushort(__hneg(mid)) << 16);
         w1 = (uint32_t)__bfloat16_as_ushort(__hneg(lo));
       }
-      // chunks 0 and 1 of the row carry the 16 columns of the k-step; the rest of the 128-byte row is unused
-      *reinterpret_cast<uint4*>(kx + swz(r, 0)) = kv0;
-      *reinterpret_cast<uint4*>(kx + swz(r, 1)) = make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(qx + swz(r, 0)) = make_uint4(w0, w1, 0, 0);
-      *reinterpret_cast<uint4*>(qx + swz(r, 1)) = make_uint4(0, 0, 0, 0);
-      fence_proxy_async_smem();
-      mbar_arrive(bar(BAR_Q_FULL));                      // release: the plain stores above
+      // two chunks of the row carry the 16 columns of a k-step
+      *reinterpret_cast<uint4*>(xt + swz(r, 0)) = kv0;
+      *reinterpret_cast<uint4*>(xt + swz(r, 1)) = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(xt + swz(r, 2)) = make_uint4(w0, w1, 0, 0);
+      *reinterpret_cast<uint4*>(xt + swz(r, 3)) = make_uint4(0, 0, 0, 0);
       // Q rows (through the permutation if given)
       int src = -1;
       if (r < rows_valid) {
@@ -302,8 +302,10 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
           else cp_async16_zfill(dst, p.q, 0);
         }
       }
-      cp_async_arrive_noinc(bar(BAR_Q_FULL));
     }
+    fence_proxy_async_smem();
+    mbar_arrive(bar(BAR_Q_FULL));                        // release: the plain stores above
+    cp_async_arrive_noinc(bar(BAR_Q_FULL));
     // ---- key tiles: contiguous rows t*128 .. t*128+127 of this head
     int n_tiles_cp = n_tiles;       // tiles copied with cp.async (none when TMA is used)
     const uint8_t* kb = reinterpret_cast<const uint8_t*>(p.k) + 2 * ((size_t)b * p.k_stride[0] + (size_t)h * p.k_stride[2]) + cch * 16;
@@ -339,9 +341,9 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       if (wrapped) ok = mbar_wait(bar(BAR_EMPTY + slot), phase ^ 1, p.status, 44);
       if (!ok) break;
       const uint32_t dst0 = sRing(slot);
-#pragma unroll
-      for (int i = 0; i < 32 / kRowsPerInstr; ++i) {
-        const int rl = row0 + i * kRowsPerInstr + sub;
+#pragma unroll 4
+      for (int i = pw; i < 128 / kRowsPerInstr; i += kProducerWarps) {
+        const int rl = i * kRowsPerInstr + sub;
         const int krow = t * kTile + rl;
         const uint32_t dst = dst0 + swz(rl, cch);
         if (c_in_tile) {

@@ -42,7 +42,7 @@ struct alignas(64) DenseTileMaps {
   unsigned long long v[16];
   int k_pos_h, k_pos_row, k_pos_b;
   int v_pos_h, v_pos_row, v_pos_b;
-  int valid;     // 0: maps not built, the dense mode gathers rows with cp.async like the sparse mode
+  int valid;
 };
 
 // (tensor_map.cu) 4-D tensor map of a (B, S, H, D) tensor of 16-bit elements with element strides {batch, row,
@@ -118,6 +118,10 @@ int launch_topk_select(const TopkParams& p, cudaStream_t stream);
 int launch_group_mass(const GroupMassParams& p, bool fp16, cudaStream_t stream);
 int launch_gather_attn_16bit(const GatherAttnParams& p, bool fp16, cudaStream_t stream);
 int launch_gather_attn_e4m3(const GatherAttnParams& p, cudaStream_t stream);
+// dense mode at head dimensions 64 and 128 (dense_attn.cu): the maps of K and V (false: a layout that no map describes),
+// and the launch
+bool dense_tile_maps(const GatherAttnParams& p, DenseTileMaps& maps);
+int launch_dense_attn(const GatherAttnParams& p, const DenseTileMaps& maps, bool fp16, cudaStream_t stream);
 // measurement aid: the K/V row gather of a sparse launch alone (gather_attn.cu)
 int launch_gather_rate_probe(const GatherAttnParams& p, int elem_bytes, cudaStream_t stream);
 // head dimensions other than 64 and 128 (multiples of 8 up to 256), bf16 / fp16 (gather_attn_wide.cu)

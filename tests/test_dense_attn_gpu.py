@@ -54,3 +54,28 @@ def test_dense_argument_errors(cuda_device):
     qh = q.to(torch.bfloat16)
     with pytest.raises(ValueError):
         full_attention(qh, qh[:, :1], qh)              # head count mismatch
+
+
+# edges of the two-stream kernel: one row, one key, stream B empty / one row, several items per CTA; and layouts that no
+# tensor map describes (keys shared by all heads: stride 0), which take the gathering kernel
+@pytest.mark.parametrize("Lq,Lk,D,shared", [(1, 1, 128, False), (128, 129, 64, False), (129, 127, 128, False), (256, 640, 64, False),
+                                            (513, 300, 128, False), (5000, 200, 64, False), (300, 260, 128, True), (257, 130, 64, True)])
+def test_dense_edges(cuda_device, Lq, Lk, D, shared):
+    from mcsparse_b200.kernels.flash_mcsa.ops.full_attn import full_attention_with_lse
+    B, H = (1, 18) if Lq == 5000 else (2, 3)
+    g = torch.Generator().manual_seed(Lq + Lk)
+    q = torch.randn(B, H, Lq, D, generator=g).to(torch.bfloat16)
+    k = (torch.randn(B, 1 if shared else H, Lk, D, generator=g) * torch.linspace(0.2, 3.0, Lk).view(1, 1, Lk, 1)).to(torch.bfloat16)
+    v = torch.randn(B, H, Lk, D, generator=g).to(torch.bfloat16)
+    perm = torch.stack([torch.randperm(Lq, generator=g) for _ in range(B * H)])
+    kd = k.to(cuda_device)
+    if shared:
+        k, kd = k.expand(B, H, Lk, D), kd.expand(B, H, Lk, D)
+    ref, ref_lse = dense_attn_ref(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2))
+    out, lse = full_attention_with_lse(q.to(cuda_device), kd, v.to(cuda_device), perm=perm.to(cuda_device))
+    mx, mr = error_metrics(out.float().cpu().transpose(1, 2), ref)
+    assert mx < 2e-2 and mr < 1e-2, (mx, mr)
+    assert float((lse.cpu() - ref_lse).abs().max()) < 2e-3
+    out_g, lse_g = full_attention_with_lse(q.to(cuda_device), kd, v.to(cuda_device), perm=perm.to(cuda_device), group_order=True)
+    idx = perm.view(B, H, Lq).to(cuda_device)
+    assert torch.equal(out_g, out.gather(2, idx.unsqueeze(-1).expand_as(out))) and torch.equal(lse_g, lse.gather(2, idx))

@@ -277,6 +277,19 @@ int mcs_topk_select_var(const float* scores, int32_t* out, const int32_t* sinks,
  * Replaces: the sort + cumulative sum + mask count of mcsparse/kernels/flash_mcsa/token_sparse.py:842-852 and
  * :862-866 (topp / topk_topp modes); the tile alignment and the lower bound of topk_topp stay on the host.
  */
+/* The same two with the sink positions in host memory (read during the call; each in [0, L)): no copy to the device.
+ * k_rows may be NULL. */
+int mcs_topk_select_host_sinks(const float* scores, int32_t* out, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L,
+                               int32_t k_total, const int32_t* k_rows, void* stream);
+int mcs_topp_count_host_sinks(const float* scores, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
+                              int32_t* counts, void* stream);
+/*
+ * Budgets of the variable-length modes (token_sparse.py:811-823, :902-923) from ranked counts, all in device memory: per row
+ * max(base, floor_rows or floor_all, 1) in whole tiles (at most L), plus the sinks, in whole tiles again; budgets in
+ * tokens, tiles = budgets / tile, k_max = the largest budget.
+ */
+int mcs_selection_budgets(const int32_t* base, const int32_t* floor_rows, int32_t floor_all, int64_t rows, int32_t L, int32_t n_sink,
+                          int32_t tile, int32_t* budgets, int32_t* tiles, int32_t* k_max, void* stream);
 int mcs_topp_count(const float* scores, const int32_t* sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
                    int32_t* counts, void* stream);
 

@@ -40,6 +40,9 @@ EXPORTED_SYMBOLS = (
     "mcs_index_pack17",
     "mcs_index_unpack17",
     "mcs_topp_count",
+    "mcs_topk_select_host_sinks",
+    "mcs_topp_count_host_sinks",
+    "mcs_selection_budgets",
     "mcs_pddp_workspace_bytes",
     "mcs_pddp_start_vector_rows",
     "mcs_pddp_levels",
@@ -162,6 +165,14 @@ def lib() -> C.CDLL:
     L.mcs_index_unpack17.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
     L.mcs_topp_count.restype = C.c_int
     L.mcs_topp_count.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32, C.c_float, C.c_void_p, C.c_void_p]
+    L.mcs_topk_select_host_sinks.restype = C.c_int
+    L.mcs_topk_select_host_sinks.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32, C.c_int32, C.c_void_p,
+                                             C.c_void_p]
+    L.mcs_topp_count_host_sinks.restype = C.c_int
+    L.mcs_topp_count_host_sinks.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32, C.c_float, C.c_void_p, C.c_void_p]
+    L.mcs_selection_budgets.restype = C.c_int
+    L.mcs_selection_budgets.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,
+                                        C.c_void_p, C.c_void_p, C.c_void_p]
     L.mcs_pddp_workspace_bytes.restype = C.c_int64
     L.mcs_pddp_workspace_bytes.argtypes = [C.c_int32] * 3
     L.mcs_pddp_start_vector_rows.restype = C.c_int64

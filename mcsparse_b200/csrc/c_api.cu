@@ -25,6 +25,16 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 static long long* g_clock_out = nullptr;
 
+// copies a host list of sink positions into the launch's argument block; false if one lies outside the row
+static bool sink_list(const int32_t* host_sinks, int n, int L, mcs::SinkList& out) {
+  if (host_sinks == nullptr) return true;
+  for (int i = 0; i < n; ++i) {
+    if (host_sinks[i] < 0 || host_sinks[i] >= L) return false;
+    out.idx[i] = host_sinks[i];
+  }
+  return true;
+}
+
 extern "C" {
 
 void mcs_set_clock_buffer(int64_t* buf3) { g_clock_out = reinterpret_cast<long long*>(buf3); }
@@ -236,13 +246,24 @@ int mcs_group_mass(const mcs_group_mass_args* a, void* stream) {
   return mcs::launch_group_mass(p, a->dtype == MCS_DTYPE_FP16, static_cast<cudaStream_t>(stream));
 }
 
+static int topk_select(const float* scores, int32_t* out, const int32_t* sinks, const int32_t* host_sinks, int32_t n_sink, int64_t rows,
+                       int32_t L, int32_t k_total, const int32_t* k_rows, void* stream) {
+  if (scores == nullptr || out == nullptr || (n_sink > 0 && sinks == nullptr && host_sinks == nullptr)) return MCS_ERR_NULL_POINTER;
+  if (rows < 0 || L < 1 || n_sink < 0 || n_sink > mcs::kMaxSinks || k_total < n_sink || k_total > L) return MCS_ERR_BAD_SHAPE;
+  if (rows == 0) return 0;
+  mcs::TopkParams p{scores, out, sinks, (long long)rows, L, k_total, n_sink, k_rows, {}};
+  if (!sink_list(host_sinks, n_sink, L, p.sink_list)) return MCS_ERR_BAD_SHAPE;
+  return mcs::launch_topk_select(p, static_cast<cudaStream_t>(stream));
+}
+
 int mcs_topk_select(const float* scores, int32_t* out, const int32_t* sinks, int32_t n_sink, int64_t rows,
                     int32_t L, int32_t k_total, void* stream) {
-  if (scores == nullptr || out == nullptr || (n_sink > 0 && sinks == nullptr)) return MCS_ERR_NULL_POINTER;
-  if (rows < 0 || L < 1 || n_sink < 0 || n_sink > 64 || k_total < n_sink || k_total > L) return MCS_ERR_BAD_SHAPE;
-  if (rows == 0) return 0;
-  mcs::TopkParams p{scores, out, sinks, (long long)rows, L, k_total, n_sink, nullptr};
-  return mcs::launch_topk_select(p, static_cast<cudaStream_t>(stream));
+  return topk_select(scores, out, sinks, nullptr, n_sink, rows, L, k_total, nullptr, stream);
+}
+
+int mcs_topk_select_host_sinks(const float* scores, int32_t* out, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L,
+                               int32_t k_total, const int32_t* k_rows, void* stream) {
+  return topk_select(scores, out, nullptr, host_sinks, n_sink, rows, L, k_total, k_rows, stream);
 }
 
 int mcs_index_pack17(const int32_t* gi, int64_t n, uint16_t* lo, uint32_t* hi, void* stream) {
@@ -259,19 +280,36 @@ int mcs_index_unpack17(const uint16_t* lo, const uint32_t* hi, int64_t n, int32_
 
 int mcs_topk_select_var(const float* scores, int32_t* out, const int32_t* sinks, int32_t n_sink, int64_t rows, int32_t L,
                         int32_t k_max, const int32_t* k_rows, void* stream) {
-  if (scores == nullptr || out == nullptr || k_rows == nullptr || (n_sink > 0 && sinks == nullptr)) return MCS_ERR_NULL_POINTER;
-  if (rows < 0 || L < 1 || n_sink < 0 || n_sink > 64 || k_max < n_sink || k_max > L) return MCS_ERR_BAD_SHAPE;
-  if (rows == 0) return 0;
-  mcs::TopkParams p{scores, out, sinks, (long long)rows, L, k_max, n_sink, k_rows};
-  return mcs::launch_topk_select(p, static_cast<cudaStream_t>(stream));
+  if (k_rows == nullptr) return MCS_ERR_NULL_POINTER;
+  return topk_select(scores, out, sinks, nullptr, n_sink, rows, L, k_max, k_rows, stream);
+}
+
+static int topp_count(const float* scores, const int32_t* sinks, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
+                      int32_t* counts, void* stream) {
+  if (scores == nullptr || counts == nullptr || (n_sink > 0 && sinks == nullptr && host_sinks == nullptr)) return MCS_ERR_NULL_POINTER;
+  if (rows < 0 || L < 1 || n_sink < 0 || n_sink > mcs::kMaxSinks || n_sink >= L) return MCS_ERR_BAD_SHAPE;
+  if (!(topp > 0.f) || !(topp <= 1.f)) return MCS_ERR_BAD_SCALE;
+  mcs::SinkList list{};
+  if (!sink_list(host_sinks, n_sink, L, list)) return MCS_ERR_BAD_SHAPE;
+  return mcs::launch_topp_count(scores, sinks, list, n_sink, (long long)rows, L, topp, counts, static_cast<cudaStream_t>(stream));
 }
 
 int mcs_topp_count(const float* scores, const int32_t* sinks, int32_t n_sink, int64_t rows, int32_t L, float topp, int32_t* counts,
                    void* stream) {
-  if (scores == nullptr || counts == nullptr || (n_sink > 0 && sinks == nullptr)) return MCS_ERR_NULL_POINTER;
-  if (rows < 0 || L < 1 || n_sink < 0 || n_sink > 64 || n_sink >= L) return MCS_ERR_BAD_SHAPE;
-  if (!(topp > 0.f) || !(topp <= 1.f)) return MCS_ERR_BAD_SCALE;
-  return mcs::launch_topp_count(scores, sinks, n_sink, (long long)rows, L, topp, counts, static_cast<cudaStream_t>(stream));
+  return topp_count(scores, sinks, nullptr, n_sink, rows, L, topp, counts, stream);
+}
+
+int mcs_topp_count_host_sinks(const float* scores, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
+                              int32_t* counts, void* stream) {
+  return topp_count(scores, nullptr, host_sinks, n_sink, rows, L, topp, counts, stream);
+}
+
+int mcs_selection_budgets(const int32_t* base, const int32_t* floor_rows, int32_t floor_all, int64_t rows, int32_t L, int32_t n_sink,
+                          int32_t tile, int32_t* budgets, int32_t* tiles, int32_t* k_max, void* stream) {
+  if (base == nullptr || budgets == nullptr || tiles == nullptr || k_max == nullptr) return MCS_ERR_NULL_POINTER;
+  if (rows < 1 || L < 1 || n_sink < 0 || tile < 1 || floor_all < 0) return MCS_ERR_BAD_SHAPE;
+  return mcs::launch_selection_budgets(base, floor_rows, floor_all, (long long)rows, L, n_sink, tile, budgets, tiles, k_max,
+                                       static_cast<cudaStream_t>(stream));
 }
 
 int64_t mcs_pddp_workspace_bytes(int32_t BH, int32_t N, int32_t C) { return (int64_t)mcs::pddp_workspace_bytes(BH, N, C); }

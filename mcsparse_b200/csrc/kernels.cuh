@@ -101,18 +101,25 @@ void* pddp_static_scratch_address();
 int launch_perm_rows(const void* x, void* out, const long long* perm, int BH, int L, int row_bytes, long long x_bh,
                      long long x_row, long long o_bh, long long o_row, bool invert, cudaStream_t stream);
 
+// Sink tokens by value: a launch then needs no copy of the list to the device (and no wait for that copy).
+constexpr int kMaxSinks = 64;
+struct SinkList { int32_t idx[kMaxSinks]; };
+
 struct TopkParams {
   const float* scores;   // (rows, L)
   int32_t* out;          // (rows, k_total) ascending
-  const int32_t* sinks;  // n_sink distinct indices in [0, L)
+  const int32_t* sinks;  // n_sink distinct indices in [0, L); null: sink_list
   long long rows;
   int L, k_total, n_sink;
   const int32_t* k_rows;  // optional per-row budgets (sinks included), clamped to [n_sink, k_total]; entries beyond are zeroed
+  SinkList sink_list;
 };
 int launch_index_pack17(const int32_t* gi, long long n, uint16_t* lo, uint32_t* hi, cudaStream_t stream);
 int launch_index_unpack17(const uint16_t* lo, const uint32_t* hi, long long n, int32_t* gi, cudaStream_t stream);
-int launch_topp_count(const float* scores, const int32_t* sinks, int n_sink, long long rows, int L, float topp, int32_t* counts,
-                      cudaStream_t stream);
+int launch_topp_count(const float* scores, const int32_t* sinks, const SinkList& sink_list, int n_sink, long long rows, int L, float topp,
+                      int32_t* counts, cudaStream_t stream);
+int launch_selection_budgets(const int32_t* base, const int32_t* floor_rows, int floor_all, long long rows, int L, int n_sink, int tile,
+                             int32_t* budgets, int32_t* tiles, int32_t* k_max, cudaStream_t stream);
 
 int launch_topk_select(const TopkParams& p, cudaStream_t stream);
 int launch_group_mass(const GroupMassParams& p, bool fp16, cudaStream_t stream);

@@ -55,7 +55,8 @@ struct Shared {
 
 template <bool kBig>
 __global__ void __launch_bounds__(kThreads) topp_count_kernel(const float* __restrict__ scores, const int32_t* __restrict__ sinks,
-                                                             int n_sink, long long rows, int L, float topp, int32_t* __restrict__ counts) {
+                                                             const __grid_constant__ SinkList sink_list, int n_sink, long long rows, int L,
+                                                             float topp, int32_t* __restrict__ counts) {
   using S = Shared<kBig>;
   using Acc = typename S::Acc;
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kThreads) topp_count_kernel(const float* __res
       };
 #pragma unroll 8
       for (int j = tid; j < L; j += kThreads) count(__ldg(sc + j), 1u);
-      for (int i = tid; i < n_sink; i += kThreads) count(__ldg(sc + sinks[i]), 0xFFFFFFFFu);     // sinks are not ranked
+      for (int i = tid; i < n_sink; i += kThreads) count(__ldg(sc + (sinks != nullptr ? sinks[i] : sink_list.idx[i])), 0xFFFFFFFFu);   // not ranked
       __syncthreads();
       // thread t owns digits 4 t .. 4 t + 3: their counts and masses, then the totals above them
       unsigned int c[4], c_sum = 0u;
@@ -193,23 +194,68 @@ __global__ void __launch_bounds__(kThreads) topp_count_kernel(const float* __res
 }
 
 template <bool kBig>
-int launch(const float* scores, const int32_t* sinks, int n_sink, long long rows, int L, float topp, int32_t* counts, cudaStream_t stream) {
+int launch(const float* scores, const int32_t* sinks, const SinkList& sink_list, int n_sink, long long rows, int L, float topp,
+           int32_t* counts, cudaStream_t stream) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int smem = (int)sizeof(Shared<kBig>);
   if (cudaFuncSetAttribute(topp_count_kernel<kBig>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -8;
   const long long grid = rows < (long long)sms * 4 ? rows : (long long)sms * 4;
-  topp_count_kernel<kBig><<<(unsigned)grid, kThreads, smem, stream>>>(scores, sinks, n_sink, rows, L, topp, counts);
+  topp_count_kernel<kBig><<<(unsigned)grid, kThreads, smem, stream>>>(scores, sinks, sink_list, n_sink, rows, L, topp, counts);
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
 }  // namespace
 
-int launch_topp_count(const float* scores, const int32_t* sinks, int n_sink, long long rows, int L, float topp, int32_t* counts,
-                      cudaStream_t stream) {
+int launch_topp_count(const float* scores, const int32_t* sinks, const SinkList& sink_list, int n_sink, long long rows, int L, float topp,
+                      int32_t* counts, cudaStream_t stream) {
   if (rows == 0) return 0;
-  return L <= (1 << 20) ? launch<false>(scores, sinks, n_sink, rows, L, topp, counts, stream)
-                        : launch<true>(scores, sinks, n_sink, rows, L, topp, counts, stream);
+  return L <= (1 << 20) ? launch<false>(scores, sinks, sink_list, n_sink, rows, L, topp, counts, stream)
+                        : launch<true>(scores, sinks, sink_list, n_sink, rows, L, topp, counts, stream);
+}
+
+namespace {
+
+// Budgets of the variable-length modes from the ranked counts (token_sparse.py:811-823, :902-923): whole tiles of ranked
+// tokens, plus the sinks, to whole tiles again.  One CTA: the largest count of all rows bounds every row, and the rows are
+// few (one per query group).  As elementwise torch operations this was fifteen launches and two waits of the host.
+__global__ void __launch_bounds__(1024) selection_budgets_kernel(const int32_t* base, const int32_t* floor_rows, int floor_all, long long rows,
+                                                                 int L, int n_sink, int tile, int32_t* budgets, int32_t* tiles, int32_t* k_max) {
+  __shared__ int warp_max[32];
+  const int tid = threadIdx.x;
+  auto up = [&](long long v) { return (v + tile - 1) / tile * tile; };
+  auto ranked = [&](long long i) -> long long {
+    const int c = max(max(base[i], floor_rows != nullptr ? floor_rows[i] : floor_all), 1);
+    return min(up(c), (long long)L);
+  };
+  int m = 0;
+  for (long long i = tid; i < rows; i += 1024) m = max(m, (int)ranked(i));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((tid & 31) == 0) warp_max[tid >> 5] = m;
+  __syncthreads();
+  m = 0;
+  for (int w = 0; w < 32; ++w) m = max(m, warp_max[w]);
+  const long long avail = (long long)m + n_sink;            // length of [sinks, longest ranked prefix]
+  const long long cap = max((long long)tile, min(up(L), avail / tile * tile));
+  auto budget = [&](long long c) {
+    if (n_sink > 0) c = min(up(c + n_sink), avail);
+    c = min(max(c, (long long)tile), cap);
+    return (int)min(c / tile * tile, (long long)L);
+  };
+  for (long long i = tid; i < rows; i += 1024) {
+    const int b = budget(ranked(i));
+    budgets[i] = b;
+    tiles[i] = b / tile;
+  }
+  if (tid == 0) *k_max = budget(m);                          // budgets grow with the count
+}
+
+}  // namespace
+
+int launch_selection_budgets(const int32_t* base, const int32_t* floor_rows, int floor_all, long long rows, int L, int n_sink, int tile,
+                             int32_t* budgets, int32_t* tiles, int32_t* k_max, cudaStream_t stream) {
+  selection_budgets_kernel<<<1, 1024, 0, stream>>>(base, floor_rows, floor_all, rows, L, n_sink, tile, budgets, tiles, k_max);
+  return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
 }  // namespace mcs

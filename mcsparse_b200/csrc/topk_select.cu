@@ -31,7 +31,6 @@ namespace {
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
 constexpr int kHistCopies = 8;
-constexpr int kMaxSinks = 64;
 
 __device__ __forceinline__ uint32_t score_key(float s) {
   uint32_t u = __float_as_uint(s);
@@ -40,6 +39,8 @@ __device__ __forceinline__ uint32_t score_key(float s) {
   u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);          // order-preserving
   return u < 2u ? 2u : u;                                  // keep 0 (sink) and 1 (padding) reserved
 }
+
+__device__ __forceinline__ int sink_at(const TopkParams& p, int i) { return p.sinks != nullptr ? p.sinks[i] : p.sink_list.idx[i]; }
 
 struct Shared {
   uint32_t hist[kHistCopies][256];
@@ -51,14 +52,14 @@ struct Shared {
 };
 
 template <bool kStage>
-__global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const __grid_constant__ TopkParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
   uint32_t* skeys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(Shared));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int L = p.L, n_sink = p.n_sink;
 
-  if (tid < n_sink) sh.sinks[tid] = p.sinks[tid];
+  if (tid < n_sink) sh.sinks[tid] = sink_at(p, tid);
   __syncthreads();
 
 #pragma unroll 1
@@ -300,7 +301,7 @@ __device__ __forceinline__ uint32_t stream_scan_excl(SharedStream& sh, uint32_t 
 // kCtas CTAs per SM with kSU 16-byte loads per thread in flight (and as many being processed): 3 with 2 or, where a
 // row's candidates take more than a third of shared memory, 2 with 4.
 template <int kCtas, int kSU>
-__global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const TopkParams p, int cap, int words) {
+__global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_constant__ TopkParams p, int cap, int words) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   SharedStream& sh = *reinterpret_cast<SharedStream*>(smem_raw);
   uint32_t* ckeys = reinterpret_cast<uint32_t*>(smem_raw + sizeof(SharedStream));   // [cap] candidates; later the output
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const TopkParam
     for (int i = tid; i < words; i += kST) bm[i] = 0u;
     if (tid == 0) { sh.n_cand = 0u; sh.n_dead = 0u; sh.n_tie = 0u; sh.key_lo = 0xFFFFFFFFu; sh.key_hi = 0u; }
     __syncthreads();
-    if (tid < n_sink) set_bit(p.sinks[tid]);                     // until the end of the row: bit set == sink
+    if (tid < n_sink) set_bit(sink_at(p, tid));                  // until the end of the row: bit set == sink
     __syncthreads();
     auto is_sink = [&](int j) { return ((bm[j >> 5] >> (j & 31)) & 1u) != 0u; };
 
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const TopkParam
         mark(false, true);
         __syncthreads();
         if (from_row) {                                          // a sink that equals T takes no part in the ranking
-          if (tid < n_sink) atomicAnd(&bm[p.sinks[tid] >> 5], ~(1u << (p.sinks[tid] & 31)));
+          if (tid < n_sink) atomicAnd(&bm[sink_at(p, tid) >> 5], ~(1u << (sink_at(p, tid) & 31)));
           __syncthreads();
         }
         uint32_t n = 0;
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const TopkParam
         }
         __syncthreads();
         mark(true, false);
-        if (tid < n_sink) set_bit(p.sinks[tid]);
+        if (tid < n_sink) set_bit(sink_at(p, tid));
       }
       __syncthreads();
     }

@@ -10,6 +10,7 @@ that sit on the accelerated path; the compute runs in the CUDA library through t
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import math
 from typing import Optional
 
@@ -89,6 +90,11 @@ def _sink_indices(sink_ranges, L_K: int):
     return sorted(idx)
 
 
+def _sink_array(sinks):
+    """The sink positions as a ctypes array (the library copies them into the launch's arguments), or None."""
+    return (ctypes.c_int32 * len(sinks))(*sinks) if sinks else None
+
+
 def select_topk_with_sinks(scores: torch.Tensor, k_total: int, sink_ranges=None,
                            out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Exact selection: the sink tokens plus the ``k_total - n_sink`` highest-scoring other tokens.
@@ -113,11 +119,9 @@ def select_topk_with_sinks(scores: torch.Tensor, k_total: int, sink_ranges=None,
         out = torch.empty(shape, dtype=torch.int32, device=scores.device)
     elif tuple(out.shape) != shape or out.dtype != torch.int32 or not out.is_contiguous():
         raise ValueError(f"out must be a contiguous int32 tensor of shape {shape}")
-    sink_t = torch.tensor(sinks, dtype=torch.int32, device=scores.device) if sinks else None
     stream = torch.cuda.current_stream(scores.device).cuda_stream
-    rc = _lib.lib().mcs_topk_select(scores.data_ptr(), out.data_ptr(),
-                                    None if sink_t is None else sink_t.data_ptr(), len(sinks), rows, L,
-                                    int(k_total), stream)
+    rc = _lib.lib().mcs_topk_select_host_sinks(scores.data_ptr(), out.data_ptr(), _sink_array(sinks), len(sinks), rows, L,
+                                               int(k_total), None, stream)
     _lib.raise_on_error(rc, f"select_topk_with_sinks")
     if _lib.check_enabled():
         _lib.check_status(scores.device, "select_topk_with_sinks")
@@ -137,10 +141,9 @@ def topp_count(scores: torch.Tensor, topp: float, sink_ranges=None) -> torch.Ten
     scores = scores.contiguous()
     rows = scores.numel() // L
     out = torch.empty(scores.shape[:-1], dtype=torch.int32, device=scores.device)
-    sink_t = torch.tensor(sinks, dtype=torch.int32, device=scores.device) if sinks else None
     stream = torch.cuda.current_stream(scores.device).cuda_stream
-    rc = _lib.lib().mcs_topp_count(scores.data_ptr(), None if sink_t is None else sink_t.data_ptr(), len(sinks), rows, L,
-                                   float(topp), out.data_ptr(), stream)
+    rc = _lib.lib().mcs_topp_count_host_sinks(scores.data_ptr(), _sink_array(sinks), len(sinks), rows, L, float(topp),
+                                              out.data_ptr(), stream)
     _lib.raise_on_error(rc, "topp_count")
     if _lib.check_enabled():
         _lib.check_status(scores.device, "topp_count")
@@ -164,28 +167,34 @@ def select_topk_var(scores: torch.Tensor, k_rows: torch.Tensor, k_max: int, sink
     k_rows = k_rows.to(torch.int32).contiguous()
     rows = scores.numel() // L
     out = torch.empty(tuple(scores.shape[:-1]) + (k_max,), dtype=torch.int32, device=scores.device)
-    sink_t = torch.tensor(sinks, dtype=torch.int32, device=scores.device) if sinks else None
     stream = torch.cuda.current_stream(scores.device).cuda_stream
-    rc = _lib.lib().mcs_topk_select_var(scores.data_ptr(), out.data_ptr(), None if sink_t is None else sink_t.data_ptr(),
-                                        len(sinks), rows, L, int(k_max), k_rows.data_ptr(), stream)
+    rc = _lib.lib().mcs_topk_select_host_sinks(scores.data_ptr(), out.data_ptr(), _sink_array(sinks), len(sinks), rows, L,
+                                               int(k_max), k_rows.data_ptr(), stream)
     _lib.raise_on_error(rc, "select_topk_var")
     if _lib.check_enabled():
         _lib.check_status(scores.device, "select_topk_var")
     return out
 
 
-def selection_counts(L_K: int, n_sink: int, tile_n: int, base_counts: torch.Tensor) -> torch.Tensor:
+def selection_budgets(L_K: int, n_sink: int, tile_n: int, base: torch.Tensor, floor_rows: Optional[torch.Tensor] = None,
+                      floor_all: int = 0):
     """Budget arithmetic of the variable-length modes (token_sparse.py:811-823, :902-923): the per-row number of
-    ranked tokens is rounded up to whole tiles (never beyond L_K), the sinks are added, the total is rounded up to whole
-    tiles again as long as ranked tokens are left to fill it, else down, and it is at least one tile."""
-    c = base_counts.long().clamp(min=1)
-    c = (((c + tile_n - 1) // tile_n) * tile_n).clamp(max=L_K)
-    avail = int(c.max().item()) + n_sink                      # length of [sinks, ranked prefix] in the reference
-    if n_sink:
-        c = (((c + n_sink + tile_n - 1) // tile_n) * tile_n).clamp(max=avail)
-    cap = max(tile_n, min(((L_K + tile_n - 1) // tile_n) * tile_n, (avail // tile_n) * tile_n))
-    c = c.clamp(min=tile_n, max=cap)
-    return ((c // tile_n) * tile_n).clamp(max=L_K)
+    ranked tokens (at least ``floor_rows`` / ``floor_all``) is rounded up to whole tiles (never beyond L_K), the sinks are
+    added, the total is rounded up to whole tiles again as long as ranked tokens are left to fill it, else down, and it
+    is at least one tile.  ``base`` and ``floor_rows``: int32 CUDA tensors, one entry per row.  Returns budgets in
+    tokens, tile counts (both int32, shape of ``base``) and the largest budget as a number (the host waits for it: it is
+    the width of the index list)."""
+    base = base.contiguous()
+    if floor_rows is not None:
+        floor_rows = floor_rows.to(torch.int32).contiguous()
+    budgets, tiles = torch.empty_like(base), torch.empty_like(base)
+    k_max = torch.empty(1, dtype=torch.int32, device=base.device)
+    stream = torch.cuda.current_stream(base.device).cuda_stream
+    rc = _lib.lib().mcs_selection_budgets(base.data_ptr(), None if floor_rows is None else floor_rows.data_ptr(), int(floor_all),
+                                          base.numel(), L_K, n_sink, tile_n, budgets.data_ptr(), tiles.data_ptr(), k_max.data_ptr(),
+                                          stream)
+    _lib.raise_on_error(rc, "selection_budgets")
+    return budgets, tiles, int(k_max.item())
 
 
 def _select_topk_tokens(token_probs, topk_ratio, tile_n=128, ds_k=1, orig_L_K=None,
@@ -223,22 +232,20 @@ def _select_topk_tokens(token_probs, topk_ratio, tile_n=128, ds_k=1, orig_L_K=No
         lengths = torch.full((B, H, M), count // tile_n, dtype=torch.int32, device=token_probs.device)
         return gi, lengths
     # ---- every row with a budget of its own
+    floor_rows, floor_all = None, 0
     if selection_mode == 'topk':
-        base = (topk_ratio.to(scores.device).float() * L_K).long().view(B, H, 1).expand(B, H, M)
+        base = (topk_ratio.to(scores.device).float() * L_K).to(torch.int32).view(B, H, 1).expand(B, H, M)
     else:
         if topp is None:
             raise AssertionError(f"{selection_mode} mode requires topp")
-        base = topp_count(scores, topp, sink_ranges).long()
+        base = topp_count(scores, topp, sink_ranges)
         if selection_mode == 'topk_topp':
             if adaptive:
-                floor_k = (topk_ratio.to(scores.device).float() * L_K).clamp(min=1, max=L_K).long().view(B, H, 1).expand(B, H, M)
+                floor_rows = (topk_ratio.to(scores.device).float() * L_K).clamp(min=1, max=L_K).long().view(B, H, 1).expand(B, H, M)
             else:
-                floor_k = torch.full_like(base, min(max(1, int(topk_ratio * L_K)), L_K))
-            base = torch.maximum(base, floor_k)
-    counts = selection_counts(L_K, len(sinks), tile_n, base)
-    k_max = int(counts.max().item())
-    gi = select_topk_var(scores, counts.to(torch.int32), k_max, sink_ranges)
-    return gi, (counts // tile_n).to(torch.int32).contiguous()
+                floor_all = min(max(1, int(topk_ratio * L_K)), L_K)
+    budgets, tiles, k_max = selection_budgets(L_K, len(sinks), tile_n, base, floor_rows, floor_all)
+    return select_topk_var(scores, budgets, k_max, sink_ranges), tiles
 
 
 def _compute_adaptive_topk_token(token_probs, base_topk, layer_t=None):

@@ -24,6 +24,7 @@ makes around the kernel into the kernel itself:
 
 from __future__ import annotations
 
+import functools
 import math
 from typing import Optional, Tuple
 
@@ -89,9 +90,14 @@ def maybe_contiguous(x: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     return x.contiguous() if x is not None and x.stride(-1) != 1 else x
 
 
-def _get_device_arch() -> int:
-    major, minor = torch.cuda.get_device_capability()
+@functools.lru_cache(maxsize=None)
+def _device_arch(device: int) -> int:
+    major, minor = torch.cuda.get_device_capability(device)
     return major * 10 + minor
+
+
+def _get_device_arch() -> int:
+    return _device_arch(torch.cuda.current_device())
 
 
 def _validate_head_dims(head_dim: int, head_dim_v: int, alignment: int) -> None:
@@ -119,7 +125,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _check_common(q, k, v, gather_kv_indices, what: str):
-    if not torch.cuda.is_available():
+    if not q.is_cuda and not torch.cuda.is_available():    # (a CUDA tensor says that there is a device; the query itself is slow)
         raise RuntimeError("CUDA is required")
     arch = _get_device_arch()
     if arch // 10 != 10:

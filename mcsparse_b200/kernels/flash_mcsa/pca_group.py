@@ -11,6 +11,8 @@ not needed on the hot path at all.
 
 from __future__ import annotations
 
+import threading
+from collections import OrderedDict
 from typing import Optional
 
 import torch
@@ -55,6 +57,49 @@ def pddp_start_vectors(BH: int, N: int, C: int, D: int, seed: int = 0) -> Tensor
     return v
 
 
+class _StartVectorPool:
+    """Device copies of the default start vectors, which depend on nothing but (BH, N, C, D, seed): a denoising run groups
+    the queries of every layer with the same ones.  Drawing them takes the host 3.4 ms at 24 heads x 32,760 tokens, the
+    grouping itself 1.4 ms.  Bounded (least recently used entries go first), shared by all threads, and every use is
+    recorded on the stream that reads the tensor, so an entry that is dropped stays valid until its readers are done."""
+
+    MAX_ENTRIES, MAX_BYTES = 16, 64 << 20
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._entries = OrderedDict()
+
+    def get(self, BH: int, N: int, C: int, D: int, seed: int, device) -> Tensor:
+        key = (device.index if device.index is not None else torch.cuda.current_device(), BH, N, C, D, seed)
+        with self._lock:
+            sv = self._entries.get(key)
+            if sv is not None:
+                self._entries.move_to_end(key)
+        if sv is None:
+            # (a copy from pageable memory: complete for every stream when the call returns)
+            sv = pddp_start_vectors(BH, N, C, D, seed).to(device=device)
+            if 4 * sv.numel() <= self.MAX_BYTES:
+                with self._lock:
+                    self._entries[key] = sv
+                    self._entries.move_to_end(key)
+                    while len(self._entries) > self.MAX_ENTRIES or sum(4 * t.numel() for t in self._entries.values()) > self.MAX_BYTES:
+                        self._entries.popitem(last=False)
+        sv.record_stream(torch.cuda.current_stream(device))
+        return sv
+
+    def clear(self) -> None:
+        with self._lock:
+            self._entries.clear()
+
+
+_start_vectors = _StartVectorPool()
+
+
+def release_start_vectors() -> None:
+    """Give back the device memory of the start vectors kept between calls."""
+    _start_vectors.clear()
+
+
 @torch.no_grad()
 def pca_group_perm(x: Tensor, C: int = 128, pow_iters: int = 4, seed: int = 0, proj_dim: Optional[int] = None,
                    *, start_vectors: Optional[Tensor] = None, return_debug: bool = False):
@@ -86,8 +131,9 @@ def pca_group_perm(x: Tensor, C: int = 128, pow_iters: int = 4, seed: int = 0, p
     if ws_bytes <= 0:
         raise ValueError("sequence too long for the grouping tables")
     if start_vectors is None:
-        start_vectors = pddp_start_vectors(BH, N, C, D, seed)
-    sv = start_vectors.to(device=x.device, dtype=torch.float32).contiguous()
+        sv = _start_vectors.get(BH, N, int(C), D, int(seed), x.device)
+    else:
+        sv = start_vectors.to(device=x.device, dtype=torch.float32).contiguous()
     levels = int(L.mcs_pddp_levels(N, C))
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
     perm = torch.empty(BH, N, dtype=torch.int64, device=x.device)

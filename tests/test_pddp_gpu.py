@@ -105,3 +105,32 @@ def test_tiny_groups(cuda_device, N, C):
                                             (1, 8200, 64, 128, 4), (1, 16500, 128, 128, 4), (1, 700, 64, 32, 4)])
 def test_node_edges(cuda_device, BH, N, D, C, iters):
     test_two_stage_contract(cuda_device, BH, N, D, C, iters)
+
+
+def test_default_start_vectors_are_kept_and_given_back(cuda_device):
+    """The default start vectors are those of ``pddp_start_vectors``; they are kept between calls (bounded), usable from other
+    streams and threads, and can be released."""
+    import threading
+    from mcsparse_b200.kernels.flash_mcsa import pca_group as P
+    P.release_start_vectors()
+    x = _clustered(2, 1500, 64, 5).to(cuda_device)
+    want = P.pca_group_perm(x, start_vectors=P.pddp_start_vectors(2, 1500, 128, 64, seed=3), seed=3)
+    assert torch.equal(P.pca_group_perm(x, seed=3), want) and torch.equal(P.pca_group_perm(x, seed=3), want)
+    assert not torch.equal(P.pca_group_perm(x, seed=4), want)
+    got = [None] * 4
+
+    def work(i):
+        with torch.cuda.device(cuda_device), torch.cuda.stream(torch.cuda.Stream()):
+            for n in range(20):
+                P.pca_group_perm(x[:, : 300 + 50 * n], seed=i)          # more shapes than the pool keeps
+            got[i] = P.pca_group_perm(x, seed=3)
+            torch.cuda.current_stream().synchronize()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert all(torch.equal(g, want) for g in got)
+    assert len(P._start_vectors._entries) <= P._StartVectorPool.MAX_ENTRIES
+    P.release_start_vectors()
+    assert not P._start_vectors._entries

@@ -23,8 +23,13 @@
 //
 // What bounds it: per pair of tiles the tensor pipe needs 2,048 cycles and the special-function unit the same
 // (32,768 exponentials at 16 per clock); under a long load the GPU's power limit lowers the clock.  Measured at 24 heads x
-// 32,760 x 128 bf16 (13.2 TFLOP; 8.0 ms at the measured burst rate, 9.4 at the sustained one): 11.24 -> 10.01 ms in short
-// bursts, 12.98 -> 11.58 ms in a long loop.
+// 32,760 x 128 bf16 (13.2 TFLOP; 8.0 ms at the measured burst rate, 9.4 at the sustained one): 11.24 -> 10.14 ms in short
+// bursts, 12.98 -> 11.54 ms in a long loop (3,146 cycles per pair of tiles; 1.77 GHz in a burst, 1.51 GHz in the loop).
+// The exponentials are not what is left: without any (results wrong, timing only) a pair takes 3,225 cycles against 3,260
+// before P V started early.  Shared memory is as busy as the tensor pipe: Q K^T reads both operands from it at 128 bytes
+// per cycle, its full rate, while the next tiles are written.  Measured and not kept: an eighth / a quarter of the
+// exponentials as polynomials on the FMA pipe (12.18 / 12.19 ms against 11.67 in the loop: issue slots and energy), scalar
+// instead of two-wide fused multiply-adds (12.13), P V started at half of the tile (11.60 against 11.54 at three quarters).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -39,6 +44,7 @@ constexpr int kTileN = 128;
 constexpr int kThreadsD = 384;
 constexpr int kTmaWarp = 8, kIssueWarp = 9, kQWarp0 = 10;
 constexpr uint32_t kColS = 0, kColO = 256;
+constexpr int kEarly = 6;       // P V of a tile starts when the probabilities of its first kEarly k-steps (of 8) are stored
 
 template <int D>
 struct SmemD {
@@ -50,7 +56,7 @@ struct SmemD {
   // barriers
   static constexpr int kFull = 0, kEmpty = kRing;          // [kRing]
   static constexpr int kQFull = 2 * kRing, kQEmpty = kQFull + 2, kSFull = kQEmpty + 2, kPReady = kSFull + 2, kOFull = kPReady + 2,
-                       kOFree = kOFull + 2, kDrain = kOFree + 2, kCount = kDrain + 1;
+                       kOFree = kOFull + 2, kPEarly = kOFree + 2, kDrain = kPEarly + 2, kCount = kDrain + 1;
   static constexpr int kSlot = kBars + kCount * 8;
   static constexpr int kDynamic = kSlot + 16 + 1024;
 };
@@ -104,6 +110,7 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
       mbar_init(bar(L::kQFull + x), 32);
       mbar_init(bar(L::kQEmpty + x), 1);
       mbar_init(bar(L::kSFull + x), 1);
+      mbar_init(bar(L::kPEarly + x), 4);
       mbar_init(bar(L::kPReady + x), 4);
       mbar_init(bar(L::kOFull + x), 1);
       mbar_init(bar(L::kOFree + x), 4);
@@ -139,7 +146,8 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
 #pragma unroll 1
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       if (x == 1 && !has_b(item)) continue;
-      float m_run = -INFINITY, l_run = 0.f;
+      // the sums of the two column halves are kept apart: the order of additions of the gathering kernel, and with it its bits
+      float m_run = -INFINITY, l_run[2] = {0.f, 0.f};
 #pragma unroll 1
       for (int t = 0; t < T; ++t, ++g) {
         ok = mbar_wait(bar(L::kSFull + x), g & 1, p.status, 110);
@@ -170,7 +178,8 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
         if (__any_sync(0xffffffffu, raise)) {
           const float alpha = raise ? ex2_approx(m_run - m_loc) : 1.f;
           if (raise) m_run = m_loc;
-          l_run *= alpha;
+          l_run[0] *= alpha;
+          l_run[1] *= alpha;
           if (t > 0) {
 #pragma unroll 1
             for (int c = 0; c < D / 8; ++c) {
@@ -184,7 +193,7 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
           }
         }
         const unsigned long long neg2 = f2_pack(-m_run, -m_run);
-        unsigned long long ls[2] = {0ull, 0ull};             // two packed partial row sums
+        unsigned long long ls[2][2] = {};                    // [column half][chain] packed partial sums
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint32_t pk[8];
@@ -193,13 +202,21 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
             const int e = c * 16 + 2 * i;
             const float2 y = f2_unpack(f2_fma(f2_pack(__uint_as_float(sc[e]), __uint_as_float(sc[e + 1])), scale2, neg2));
             const float p0 = ex2_approx(y.x), p1 = ex2_approx(y.y);
-            ls[i & 1] = f2_add(ls[i & 1], f2_pack(p0, p1));
+            ls[c / 4][i & 1] = f2_add(ls[c / 4][i & 1], f2_pack(p0, p1));
             pk[i] = kFp16 ? pack_f16x2(p0, p1) : pack_bf16x2(p0, p1);
           }
           tmem_st8(tS + c * 8, pk);
+          if (c == kEarly - 1) {
+            tmem_wait_st();
+            tc_fence_before();
+            warp_arrive(bar(L::kPEarly + x));
+          }
         }
-        const float2 l2 = f2_unpack(f2_add(ls[0], ls[1]));
-        l_run += l2.x + l2.y;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2 a0 = f2_unpack(ls[q][0]), a1 = f2_unpack(ls[q][1]);
+          l_run[q] += (a0.x + a0.y) + (a1.x + a1.y);
+        }
         tmem_wait_st();
         tc_fence_before();
         warp_arrive(bar(L::kPReady + x));
@@ -224,7 +241,7 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
       ok = mbar_wait(bar(L::kOFull + x), ic & 1, p.status, 111);
       if (!ok) break;
       tc_fence_after();
-      const float w = p.out_sign / l_run;
+      const float l_all = l_run[0] + l_run[1], w = p.out_sign / l_all;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t ra[32];
@@ -258,7 +275,7 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
           }
         }
       }
-      if (valid && p.lse != nullptr) p.lse[(size_t)bh * p.Sq + orow] = (m_run + lg2_approx(l_run)) * 0.6931471805599453f;
+      if (valid && p.lse != nullptr) p.lse[(size_t)bh * p.Sq + orow] = (m_run + lg2_approx(l_all)) * 0.6931471805599453f;
       ++ic;
     }
     tc_fence_before();
@@ -331,15 +348,21 @@ __global__ void __launch_bounds__(kThreadsD, 1) dense_attn_kernel(const GatherAt
       if (last) ++iq[x];
     };
     auto pv = [&](int x, int vslot, bool first, bool last) {
-      ok = ok && mbar_wait(bar(L::kPReady + x), g[x] & 1, p.status, 114);
+      ok = ok && mbar_wait(bar(L::kPEarly + x), g[x] & 1, p.status, 114);
       if (first && ic[x] > 0) ok = ok && mbar_wait(bar(L::kOFree + x), (ic[x] - 1) & 1, p.status, 115);
       if (!ok) return;
       tc_fence_after();
       const uint32_t vlo = ((sRing(vslot) & 0x3FFFFu) >> 4) | kLboV;
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < 8; ++j) {
+        if (j == kEarly) {
+          ok = mbar_wait(bar(L::kPReady + x), g[x] & 1, p.status, 120);
+          if (!ok) return;
+          tc_fence_after();
+        }
         if (leader)
           mma_f16_ts(tmem + kColO + x * D, tmem + kColS + x * 128 + j * 8, desc(vlo + j * (2048 >> 4)), idesc_pv, !first || j > 0);
+      }
       if (leader && last) tc_commit(bar(L::kOFull + x));
       ++g[x];
       if (last) ++ic[x];

@@ -127,3 +127,17 @@ def test_topp_count_wide_range(cuda_device, L):
     tp[..., 0] = 3.0
     got = topp_count(tp.to(cuda_device), 0.609375, [(0, 1)]).cpu()
     assert torch.equal(got, topp_count_ref(tp, 0.609375, [0]).to(got.dtype)), got      # exact integer sums per bin: no rounding slack
+
+
+@pytest.mark.parametrize("L,n_sink,rows,hi", [(100, 0, 1, 100), (100, 5, 7, 100), (4096, 4, 3000, 4096), (32760, 4, 300, 32760), (640, 64, 50, 3)])
+def test_selection_budgets_match_oracle(cuda_device, L, n_sink, rows, hi):
+    from mcsparse_b200.kernels.flash_mcsa.token_sparse import selection_budgets
+    from oracle.select import selection_counts_ref
+    g = torch.Generator().manual_seed(rows)
+    base = torch.randint(0, hi + 1, (rows,), generator=g, dtype=torch.int32)
+    floor = torch.randint(1, hi + 1, (rows,), generator=g, dtype=torch.int32)
+    for fr, fa in ((None, 0), (None, min(200, L)), (floor, 0)):
+        eff = torch.maximum(base, fr if fr is not None else torch.full_like(base, fa))
+        want = selection_counts_ref(L, n_sink, 128, eff).clamp(max=L).to(torch.int32)
+        b, t, m = selection_budgets(L, n_sink, 128, base.to(cuda_device), None if fr is None else fr.to(cuda_device), fa)
+        assert torch.equal(b.cpu(), want) and torch.equal(t.cpu(), want // 128) and m == int(want.max())

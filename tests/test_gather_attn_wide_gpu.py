@@ -108,3 +108,28 @@ def test_head_dim_errors(cuda_device):
         x = torch.randn(1, 128, 1, D, device=cuda_device).to(torch.bfloat16)
         with pytest.raises(ValueError):
             flash_attn_gather_kv_func(x, x, x, gi)
+
+
+@pytest.mark.parametrize("D", [72, 96, 144, 160, 224, 256])
+def test_rising_maximum_bits_and_single_tiles(cuda_device, D):
+    """Groups of one to nine tiles whose scores grow from tile to tile (the accumulator is rescaled while products are in
+    flight), more groups than SMs, against the oracle; and the same bits on every launch."""
+    H, Sq, Sk = 3, 6600, 1400
+    g = torch.Generator().manual_seed(D)
+    dirn = torch.nn.functional.normalize(torch.randn(D, generator=g), dim=0)
+    q = (torch.randn(1, Sq, H, D, generator=g) * 0.5 + 3.0 * dirn).to(torch.float16)
+    k = (torch.randn(1, Sk, H, D, generator=g) * 0.5 + torch.linspace(0, 6.0 * math.sqrt(D), Sk).view(1, Sk, 1, 1) * dirn).to(torch.float16)
+    v = torch.randn(1, Sk, H, D, generator=g).to(torch.float16)
+    M = math.ceil(Sq / 128)
+    gi = torch.stack([torch.randperm(Sk, generator=g)[:1152].sort().values for _ in range(H * M)]).view(1, H, M, 1152).to(torch.int32)
+    gl = torch.randint(1, 10, (1, H, M), dtype=torch.int32, generator=g)
+    res = (0.1 * torch.randn(1, H, Sq, D, generator=g)).to(torch.float16)
+    out, lse = _run(cuda_device, q, k, v, gi, gather_kv_lengths=gl, residual=res)
+    for _ in range(3):
+        o2, l2 = _run(cuda_device, q, k, v, gi, gather_kv_lengths=gl, residual=res)
+        assert torch.equal(out, o2) and torch.equal(lse, l2)
+    heads = [0, H - 1]
+    ref, ref_lse = gather_attn_ref(q[:, :, heads], k[:, :, heads], v[:, :, heads], gi[:, heads], gl=gl[:, heads], residual=res[:, heads])
+    mx, mr = error_metrics(out[:, :, heads], ref)
+    assert mx < MAX_ABS and mr < MEAN_REL, (mx, mr)
+    assert (lse[:, heads] - ref_lse).abs().max() < 2e-2

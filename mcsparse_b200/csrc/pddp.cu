@@ -742,22 +742,27 @@ __global__ void __launch_bounds__(256) pddp_wide_project_kernel(PddpParams p, in
 // ------------------------------------------------------------------------------------------
 // sort: bitonic network over segments of `pad` keys (power of two), ascending inside each segment
 // ------------------------------------------------------------------------------------------
-// A CTA sorts kSortTile consecutive slots (several short segments or a part of a long one) out of registers: thread t
-// holds slots 8 t .. 8 t + 7, so distances below 8 stay inside a thread, distances 8 to 128 are lane exchanges and only
-// those of 256 and more (10 of the 78 steps of a full tile) go through shared memory.  All 14 sorts and 8 scatters of the call
-// above: 560 us with every step in shared memory and a scatter kernel, 388 us this way.  Stages k_lo .. k_hi; distances above the tile are done by the global kernel.
+// A CTA of kT threads sorts 8 kT consecutive slots (several short segments or a part of a long one).  A thread holds eight
+// slots whose positions differ in three neighbouring bits, b .. b + 2, and does the three compare distances of these bits in
+// registers; between groups of three the slots change hands through shared memory (padded by one slot in eight, so that
+// every layout is read and written without bank conflicts).  A full tile changes hands 27 times for its 78 steps; with the
+// distances of 8 to 128 as lane exchanges (sixteen 32-bit shuffles per step) and the larger ones through shared memory one by
+// one it took 47 us instead of 37.  Stages k_lo .. k_hi; distances above the tile are done by the global kernel.
 // The kernel of a segment's last stage writes the new order itself: new_perm[start + r] = old_perm[start + position].
+// Segments of up to 1,024 slots take CTAs of 128 threads and those of 2,048 of 256, so that a level's slots spread over more
+// CTAs than SMs.
 constexpr int kSortThreads = kSortTile / 8;
 
-__device__ __forceinline__ unsigned long long u64_min(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
-__device__ __forceinline__ unsigned long long u64_max(unsigned long long a, unsigned long long b) { return a < b ? b : a; }
-
-__global__ void __launch_bounds__(kSortThreads) pddp_sort_kernel(PddpParams p, int lv, long long slots, int pad, int k_lo, int k_hi,
-                                                                const int* perm_in, int* perm_out) {
-  __shared__ unsigned long long sk[8][kSortThreads];
+template <int kT>
+__global__ void __launch_bounds__(kT) pddp_sort_kernel(PddpParams p, int lv, long long slots, int pad, int k_lo, int k_hi,
+                                                      const int* perm_in, int* perm_out) {
+  constexpr int kTile = 8 * kT;
+  constexpr int kTileBits = kT == 128 ? 10 : (kT == 256 ? 11 : 12);
+  static_assert((1 << kTileBits) == kTile, "tile size");
+  __shared__ unsigned long long sk[kTile + kTile / 8];
   unsigned long long* keys = p.keys + (size_t)blockIdx.y * p.key_stride;
   const int tid = threadIdx.x;
-  const long long slot0 = (long long)blockIdx.x * kSortTile + tid * 8;     // slots is a multiple of 8 (pad >= 8)
+  const long long slot0 = (long long)blockIdx.x * kTile + tid * 8;         // slots is a multiple of 8 (pad >= 8)
   const bool live = slot0 < slots;
   unsigned long long a[8];
   if (live) {
@@ -769,46 +774,51 @@ __global__ void __launch_bounds__(kSortThreads) pddp_sort_kernel(PddpParams p, i
     for (int i = 0; i < 8; ++i) a[i] = 0xFFFFFFFFFFFFFFFFull;
   }
   auto cmpx = [&](int i, int j, bool asc) {
-    const unsigned long long lo = u64_min(a[i], a[j]), hi = u64_max(a[i], a[j]);
-    a[i] = asc ? lo : hi;
-    a[j] = asc ? hi : lo;
+    const bool swap = (a[i] > a[j]) == asc;
+    const unsigned long long x = swap ? a[j] : a[i], y = swap ? a[i] : a[j];
+    a[i] = x;
+    a[j] = y;
   };
-  const int gi = (int)(slot0 & (pad - 1));                                 // position of this thread's first key in its segment
+  // compare distances of bits b + 2 (if n == 3), b + 1 (if n >= 2) and b, all in one direction
+  auto steps = [&](int n, bool asc) {
+    if (n == 3) { cmpx(0, 4, asc); cmpx(1, 5, asc); cmpx(2, 6, asc); cmpx(3, 7, asc); }
+    if (n >= 2) { cmpx(0, 2, asc); cmpx(1, 3, asc); cmpx(4, 6, asc); cmpx(5, 7, asc); }
+    cmpx(0, 1, asc); cmpx(2, 3, asc); cmpx(4, 5, asc); cmpx(6, 7, asc);
+  };
+  // position in the tile of this thread's slot 0 when its slots differ in bits b .. b + 2
+  auto first = [&](int b) { return ((tid >> b) << (b + 3)) | (tid & ((1 << b) - 1)); };
+  int cur = 0;                                                             // the layout's b
+  auto relayout = [&](int b) {
+    const int f = first(cur), t = first(b);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { const int x = f + (i << cur); sk[x + (x >> 3)] = a[i]; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { const int x = t + (i << b); a[i] = sk[x + (x >> 3)]; }
+    __syncthreads();
+    cur = b;
+  };
   if (k_lo == 2) {
     cmpx(0, 1, true); cmpx(2, 3, false); cmpx(4, 5, true); cmpx(6, 7, false);
     cmpx(0, 2, true); cmpx(1, 3, true); cmpx(4, 6, false); cmpx(5, 7, false);
     cmpx(0, 1, true); cmpx(2, 3, true); cmpx(4, 5, false); cmpx(6, 7, false);
   }
+  const int tile0 = (int)(((long long)blockIdx.x * kTile) & (pad - 1));    // the tile's position inside its segment (0 if it holds several)
 #pragma unroll 1
   for (int k = max(k_lo, 8); k <= k_hi; k <<= 1) {
-    const bool asc = (k == pad) || ((gi & k) == 0);
+    int left = min(31 - __clz(k), kTileBits);                              // compare distances of bits left - 1 .. 0 are to be done
 #pragma unroll 1
-    for (int j = min(k >> 1, kSortTile >> 1); j >= 8; j >>= 1) {
-      const int m = j >> 3;                                                // distance in threads
-      const bool take_min = ((tid & m) == 0) == asc;
-      if (m >= 32) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sk[i][tid] = a[i];
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const unsigned long long b = sk[i][tid ^ m];
-          a[i] = take_min ? u64_min(a[i], b) : u64_max(a[i], b);
-        }
-        __syncthreads();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const unsigned long long b = __shfl_xor_sync(0xffffffffu, a[i], m);
-          a[i] = take_min ? u64_min(a[i], b) : u64_max(a[i], b);
-        }
-      }
+    while (left > 3) {
+      const int b = left - 3;
+      relayout(b);
+      steps(3, (k == pad) || (((tile0 + first(b)) & (pad - 1) & k) == 0)); // (bit k of the position is the same for all eight slots)
+      left = b;
     }
-    cmpx(0, 4, asc); cmpx(1, 5, asc); cmpx(2, 6, asc); cmpx(3, 7, asc);
-    cmpx(0, 2, asc); cmpx(1, 3, asc); cmpx(4, 6, asc); cmpx(5, 7, asc);
-    cmpx(0, 1, asc); cmpx(2, 3, asc); cmpx(4, 5, asc); cmpx(6, 7, asc);
+    if (cur != 0) relayout(0);
+    steps(left, (k == pad) || (((tile0 + tid * 8) & (pad - 1) & k) == 0));
   }
   if (!live) return;
+  const int gi = (int)(slot0 & (pad - 1));                                 // position of this thread's first key in its segment
   if (k_hi == pad) {
     const LevelTables T = level_tables(p.tables, lv, p.table_stride);
     const int node = (int)(slot0 / pad);
@@ -979,12 +989,16 @@ int launch_pddp(const PddpArgs& a, cudaStream_t stream) {
       v0 += (size_t)BH * ls.nodes * a.D;
       // bitonic sort of every segment of `pad` keys; the last kernel writes the new order
       const int tile_k = std::min(ls.pad, kSortTile);
-      const dim3 sgrid((unsigned)((slots + kSortTile - 1) / kSortTile), BH);
-      pddp_sort_kernel<<<sgrid, kSortThreads, 0, stream>>>(p, lv, slots, ls.pad, 2, tile_k, perm_a, perm_b);
+      auto sort = [&](auto kern, int threads, int k_lo, int k_hi) {
+        kern<<<dim3((unsigned)((slots + 8 * threads - 1) / (8 * threads)), BH), threads, 0, stream>>>(p, lv, slots, ls.pad, k_lo, k_hi, perm_a, perm_b);
+      };
+      if (ls.pad <= 1024) sort(pddp_sort_kernel<128>, 128, 2, tile_k);
+      else if (ls.pad <= 2048) sort(pddp_sort_kernel<256>, 256, 2, tile_k);
+      else sort(pddp_sort_kernel<kSortThreads>, kSortThreads, 2, tile_k);
       for (int k = tile_k * 2; k <= ls.pad; k <<= 1) {
         for (int j = k >> 1; j >= kSortTile; j >>= 1)
           pddp_sort_global_kernel<<<dim3((unsigned)((slots / 2 + 255) / 256), BH), 256, 0, stream>>>(p.keys, p.key_stride, slots / 2, ls.pad, k, j);
-        pddp_sort_kernel<<<sgrid, kSortThreads, 0, stream>>>(p, lv, slots, ls.pad, k, k, perm_a, perm_b);
+        sort(pddp_sort_kernel<kSortThreads>, kSortThreads, k, k);
       }
       std::swap(perm_a, perm_b);
     }

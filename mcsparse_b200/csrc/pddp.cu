@@ -330,6 +330,8 @@ __global__ void __launch_bounds__(kNodeThreads, 2) pddp_node_kernel(PddpParams p
     const size_t row_bytes = 2 * (size_t)p.x_stride_row;
     const int* ids = perm_in + (size_t)bh * p.N + pos0;
     bool ok = true;
+    // (in flight under the gather)
+    const float v_start = (size <= kChunkRows && tid < D) ? v0[((size_t)bh * nodes + node) * D + tid] : 0.f;
     {
       int id_next = tid < rows ? ids[tid] : -1;
       int buf = 0, phase = 0;
@@ -373,12 +375,17 @@ __global__ void __launch_bounds__(kNodeThreads, 2) pddp_node_kernel(PddpParams p
         named_bar_sync(1, 128);
         const float inv_n = 1.f / (float)size;
 #pragma unroll 1
-        for (int c = 0; c < D / 8; ++c) {
-          tmem_ld8(tmem + lane_addr + c * 8, r8);
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem + lane_addr + c * 32, r);
           tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) r8[i] = __float_as_uint(__uint_as_float(r8[i]) - ssum[c * 8 + i] * s_d * inv_n);
-          tmem_st8(tmem + lane_addr + c * 8, r8);
+          for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              r8[i] = __float_as_uint(__uint_as_float(r[q * 8 + i]) - ssum[c * 32 + q * 8 + i] * s_d * inv_n);
+            tmem_st8(tmem + lane_addr + c * 32 + q * 8, r8);
+          }
         }
         tmem_wait_st();
         // ---- power iterations
@@ -388,7 +395,7 @@ __global__ void __launch_bounds__(kNodeThreads, 2) pddp_node_kernel(PddpParams p
           named_bar_sync(1, 128);
           return (red[0] + red[1]) + (red[2] + red[3]);
         };
-        float v = d < D ? v0[((size_t)bh * nodes + node) * D + d] : 0.f;
+        float v = v_start;
         float nrm = sqrtf(sum_128(v * v));
         v /= fmaxf(nrm, 1e-12f);
         for (int iter = 0; iter < p.pow_iters; ++iter) {

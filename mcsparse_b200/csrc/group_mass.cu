@@ -10,8 +10,8 @@
 // (mcsparse/kernels/flash_mcsa/ops/triton/block_probs.py:27-89), with an fp32 result instead
 // of one rounded to bf16.
 //
-// One CTA per (batch*head, group).  The 128 query rows of the group stay resident in shared
-// memory; the CTA streams all key tiles of the head.  The product is computed TRANSPOSED,
+// One CTA per (batch*head, group), or per two neighbouring groups and a stretch of the key tiles (launch_group_mass).  The
+// query rows stay resident in shared memory; the CTA streams its key tiles of the head.  The product is computed TRANSPOSED,
 // S^T = K_tile Q^T, so that a TMEM lane is a key token and the sum over the group's queries
 // runs along the columns inside one thread: no cross-thread reduction at all.
 //
@@ -22,8 +22,8 @@
 // The kernel is bound by the ex2 throughput of the SFU (16 per clock per SM); a quarter of the exponentials
 // are therefore evaluated by a polynomial on the FMA pipe.
 //
-// Roles: warps 0-15 exponentiate and sum, in two groups of eight for the even and the odd key tiles (two threads per key
-// token: warps w and w+4 of a group share a TMEM lane group and take 64 query columns each; the two partial sums meet in
+// Roles: warps 0-15 exponentiate and sum, in two groups of eight for the even and the odd key tiles, or for the two query
+// groups (two threads per key token: warps w and w+4 of a group share a TMEM lane group and take 64 query columns each; the two partial sums meet in
 // shared memory).  Four warps per SM sub-partition feed its SFU, and each group has two score buffers of its own, so one
 // group's waits and tensor-memory loads lie under the other's exponentials: with a single group and two buffers the SFU
 // was 64% busy (7,100 -> 6,517 us at 24 heads x 32,760 x 128, 655 -> 573 us at 8 x 16,380; floors 5,900 / 500 us of ex2
@@ -43,7 +43,7 @@ namespace {
 constexpr int kTile = 128;
 constexpr int kThreads = 640;          // five warps per SM sub-partition: 96 registers each
 constexpr int kExpWarps = 16;          // two groups of eight: even and odd key tiles
-constexpr int kBufs = 4;               // score buffers in tensor memory, two per group
+constexpr int kBufs = 4;               // score buffers of 128 columns in tensor memory
 constexpr int kProducerWarps = 3;
 constexpr int kProducerThreads = kProducerWarps * 32;
 constexpr int kMmaWarp = 16;
@@ -57,15 +57,16 @@ enum { BAR_FULL = 0, BAR_EMPTY = BAR_FULL + kRing, BAR_Q_FULL = BAR_EMPTY + kRin
 
 // D is the head dimension rounded up to the tile layouts this kernel has: 64, 128, 192 or 256 (the true head
 // dimension, any multiple of 8 up to 256, is a run-time value; rows are zero-padded on their way into shared memory)
-template <int D>
+template <int D, int G>
 struct Smem {
   static constexpr int kBlocks = D / 64;
   static constexpr int kTileBytes = kBlocks * 16384;
+  static constexpr int kQRows = 128 * G;                     // G query groups per CTA, see launch_group_mass
   static constexpr int kRingN = D == 256 ? 2 : kRing;        // key-tile slots that fit beside the query tile
-  static constexpr int kQ = 0;                              // group's query rows (B operand)
-  static constexpr int kX = kTileBytes;                     // extra k-steps, 128 rows x 128 B: chunks 0-1 K's constant
+  static constexpr int kQ = 0;                              // the groups' query rows (B operand)
+  static constexpr int kX = G * kTileBytes;                 // extra k-steps, kQRows rows x 128 B: chunks 0-1 K's constant
                                                             // (1,1,1,0...), chunks 2-3 Q's, the rest unused
-  static constexpr int kRingOff = kX + 16384;
+  static constexpr int kRingOff = kX + kQRows * 128;
   static constexpr int kBars = kRingOff + kRingN * kTileBytes;
   static constexpr int kPart = kBars + BAR_COUNT * 8;       // float [kBufs][128]: partial sums of the upper column half
   static constexpr int kTmemSlot = kPart + kBufs * 128 * 4;
@@ -73,17 +74,19 @@ struct Smem {
   static constexpr int kDynamic = kTotal + 1024;
 };
 
-static_assert(Smem<192>::kDynamic <= 232448 && Smem<256>::kDynamic <= 232448, "padded layouts must fit 227 KB");
+static_assert(Smem<128, 2>::kDynamic <= 232448 && Smem<192, 1>::kDynamic <= 232448 && Smem<256, 1>::kDynamic <= 232448, "padded layouts must fit 227 KB");
 
-__device__ __forceinline__ uint32_t swz(int row, int c) {   // 16-byte chunk c of row, 128-byte swizzle
-  return static_cast<uint32_t>((c >> 3) * 16384 + row * 128 + (((c & 7) ^ (row & 7)) << 4));
+// 16-byte chunk c of row, 128-byte swizzle, tiles of kRows rows
+template <int kRows = 128>
+__device__ __forceinline__ uint32_t swz(int row, int c) {
+  return static_cast<uint32_t>((c >> 3) * (kRows * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
 }
 
-template <int D, bool kFp16, int kPoly>
-__global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMassParams p, const __grid_constant__ KeyTileMap kmap) {
+template <int D, bool kFp16, int G>
+__global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMassParams p, const __grid_constant__ KeyTileMap kmap, int splits) {
   // key tiles are 128 consecutive rows: with a valid tensor map one elected thread loads them by TMA
   const bool use_tma = kmap.valid != 0;
-  using L = Smem<D>;
+  using L = Smem<D, G>;
   constexpr bool kWide = D > 128;                       // padded layouts: the true head dimension is p.D < D
   constexpr int R = L::kRingN;
   const int d_chunks = p.D / 8;                          // 16-byte chunks of a real row
@@ -97,12 +100,16 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // provably warp-uniform
 
-  const int m = blockIdx.x % p.M;
-  const int bh = blockIdx.x / p.M;
+  // work item: a group (or two neighbouring ones) of one (batch, head) and one of `splits` stretches of its key tiles
+  const int sets = (p.M + G - 1) / G;
+  const int split = blockIdx.x % splits, set = blockIdx.x / splits;
+  const int m0 = set % sets * G;
+  const int bh = set / sets;
   const int h = bh % p.H, b = bh / p.H;
-  const int row_base = m * p.group_rows;
-  const int rows_valid = min(p.group_rows, p.Lq - row_base);
-  const int n_tiles = (p.Lk + kTile - 1) / kTile;
+  const int all_tiles = (p.Lk + kTile - 1) / kTile;
+  const int tile0 = static_cast<int>((long long)all_tiles * split / splits);
+  const int n_tiles = static_cast<int>((long long)all_tiles * (split + 1) / splits) - tile0;
+  auto rows_of = [&](int m) { return m < p.M ? min(p.group_rows, p.Lq - m * p.group_rows) : 0; };
 
   if (tid == 0) {
     for (int i = 0; i < R; ++i) {
@@ -112,7 +119,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
     mbar_init(bar(BAR_Q_FULL), 2 * kProducerThreads);   // per thread: its cp.async rows + its plain stores
     for (int i = 0; i < kBufs; ++i) {
       mbar_init(bar(BAR_S_FULL + i), 1);
-      mbar_init(bar(BAR_S_FREE + i), kExpWarps / 2);
+      mbar_init(bar(BAR_S_FREE + i), G == 2 ? kExpWarps : kExpWarps / 2);
     }
     for (int i = 0; i < 4 * kBufs; ++i) mbar_init(bar(BAR_PART + i), 1);
     mbar_init(bar(BAR_DRAIN), 1);
@@ -134,13 +141,19 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
     const uint32_t lane_addr = (static_cast<uint32_t>(lg) * 32u) << 16;
     const float c = p.scale_log2;
     const float xmin = -125.f / c;
-    const float norm = p.normalize ? 1.f / static_cast<float>(rows_valid) : 1.f;
-    float* out = p.mass + ((size_t)bh * p.M + m) * p.Lk;
+    // two groups: each eight warps take one group's columns of every tile (two buffers of 256 columns); one group: the
+    // even and the odd tiles (four buffers of 128)
+    const int eg = warp >> 3, m = G == 2 ? m0 + eg : m0;
+    const float norm = p.normalize ? 1.f / static_cast<float>(max(rows_of(m), 1)) : 1.f;
+    float* out = p.mass + ((size_t)bh * p.M + min(m, p.M - 1)) * p.Lk;
     float* part = reinterpret_cast<float*>(smem + L::kPart);
     bool ok = true;
 #pragma unroll 1
-    for (int t = warp >> 3; t < n_tiles && ok; t += 2) {
-      const int buf = t & (kBufs - 1), ph = (t / kBufs) & 1;
+    for (int t = G == 2 ? 0 : eg; t < n_tiles && ok; t += G == 2 ? 1 : 2) {
+      constexpr int kB = G == 2 ? 2 : kBufs;
+      const int buf = t & (kB - 1), ph = (t / kB) & 1;
+      const int pb = G == 2 ? 2 * eg + buf : buf;        // place of the partial sums
+      const uint32_t tS = tmem + (G == 2 ? buf * 256 + eg * 128 : buf * 128) + x * 64 + lane_addr;
       ok = mbar_wait(bar(BAR_S_FULL + buf), ph, p.status, 40);
       if (!ok) break;
       tc_fence_after();
@@ -148,18 +161,17 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         uint32_t r[32];
-        tmem_ld32(tmem + buf * 128 + x * 64 + q * 32 + lane_addr, r);
+        tmem_ld32(tS + q * 32, r);
         tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 32; i += 8) {
-          // kPoly of every eight exponentials are computed on the FMA pipe instead of the special-function unit,
-          // which bounds this kernel (see ex2_poly3_scaled); their positions are spread over the four partial sums.
-          // Two of eight measured best (6.52 ms against 6.69 / 6.88 ms with one / three at H=24, L=32,760: beyond a
+          // Two of every eight exponentials are computed on the FMA pipe instead of the special-function unit
+          // (see ex2_poly3_scaled); their positions are spread over the four partial sums.
+          // Two measured best (6.52 ms against 6.69 / 6.88 ms with one / three at H=24, L=32,760: beyond a
           // quarter the extra instructions cost more issue slots than the unit gains).
           auto e = [&](int k) {
             const float v = __uint_as_float(r[i + k]);
-            const bool poly = (kPoly >= 1 && k == 3) || (kPoly >= 2 && k == 6) || (kPoly >= 3 && k == 1) || (kPoly >= 4 && k == 4);
-            return poly ? ex2_poly3_scaled(v, c, xmin) : ex2_approx(v * c);
+            return k == 3 || k == 6 ? ex2_poly3_scaled(v, c, xmin) : ex2_approx(v * c);
           };
           a0 += e(0); a1 += e(1); a2 += e(2); a3 += e(3);
           a0 += e(4); a1 += e(5); a2 += e(6); a3 += e(7);
@@ -173,17 +185,17 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       // needs that release to get its next scores) cannot overtake the read.  (Copying all 64 values to
       // registers first and releasing the score buffer before the exponentials measured 10% slower.)
       if (x == 1) {
-        part[buf * 128 + j_in] = sum;
+        part[pb * 128 + j_in] = sum;
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(bar(BAR_PART + kBufs * lg + buf));
+          mbar_arrive(bar(BAR_PART + kBufs * lg + pb));
           mbar_arrive(bar(BAR_S_FREE + buf));              // one arrival per warp
         }
       } else {
-        ok = mbar_wait(bar(BAR_PART + kBufs * lg + buf), ph, p.status, 45);
+        ok = mbar_wait(bar(BAR_PART + kBufs * lg + pb), ph, p.status, 45);
         if (!ok) break;
-        const int j = t * kTile + j_in;
-        if (j < p.Lk) out[j] = (sum + part[buf * 128 + j_in]) * norm;
+        const int j = (tile0 + t) * kTile + j_in;
+        if (j < p.Lk && m < p.M) out[j] = (sum + part[pb * 128 + j_in]) * norm;
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(BAR_S_FREE + buf));
       }
@@ -194,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
     {
       const bool leader = elect_one();
       constexpr uint32_t kFmt = kFp16 ? 0u : 1u;
-      constexpr uint32_t idesc = mma_idesc(kFmt, kFmt, 0, 0, 128, 128);
+      constexpr uint32_t idesc = mma_idesc(kFmt, kFmt, 0, 0, 128, 128 * G);
       constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
       constexpr uint32_t kLbo = (16u >> 4) << 16;
       auto desc = [&](uint32_t lo) { return (static_cast<uint64_t>(kDescHi) << 32) | lo; };
@@ -205,13 +217,14 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       int slot = 0, phase = 0;
 #pragma unroll 1
       for (int t = 0; t < n_tiles && ok; ++t) {
-        const int buf = t & (kBufs - 1);
-        if (t >= kBufs) ok = mbar_wait(bar(BAR_S_FREE + buf), (t / kBufs - 1) & 1, p.status, 42);
+        constexpr int kB = G == 2 ? 2 : kBufs;
+        const int buf = t & (kB - 1);
+        if (t >= kB) ok = mbar_wait(bar(BAR_S_FREE + buf), (t / kB - 1) & 1, p.status, 42);
         ok = ok && mbar_wait(bar(BAR_FULL + slot), phase, p.status, 43);
         if (!ok) break;
         fence_proxy_async_smem();
         tc_fence_after();
-        const uint32_t tS = tmem + buf * 128;
+        const uint32_t tS = tmem + buf * 128 * G;
         const uint32_t klo = ((sRing(slot) & 0x3FFFFu) >> 4) | kLbo;
         if constexpr (kWide) {
           // the k-steps that hold real columns (the last one zero-padded to 16)
@@ -224,8 +237,8 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
         } else {
 #pragma unroll
           for (int j = 0; j < D / 16; ++j) {
-            const uint32_t koff = (j >> 2) * (16384 >> 4) + (j & 3) * 2;
-            if (leader) mma_f16_ss(tS, desc(klo + koff), desc(qlo + koff), idesc, j > 0);     // A = K tile, B = Q group
+            const uint32_t koff = (j >> 2) * (16384 >> 4) + (j & 3) * 2, qoff = (j >> 2) * (16384 * G >> 4) + (j & 3) * 2;
+            if (leader) mma_f16_ss(tS, desc(klo + koff), desc(qlo + qoff), idesc, j > 0);     // A = K tile, B = query rows
           }
         }
         if (leader) {
@@ -252,9 +265,9 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
     const int sub = lane / kChunks, cch = lane % kChunks;
     const bool c_in_tile = !kWide || cch < D / 8;
     const bool c_live = !kWide || cch < d_chunks;
-    // ---- constant extra K block, extra Q block, Q rows (three warps share the four blocks of 32 rows)
+    // ---- constant extra K block, extra Q block, Q rows (three warps share the blocks of 32 rows)
 #pragma unroll 1
-    for (int row0 = pw * 32; row0 < 128; row0 += kProducerThreads) {
+    for (int row0 = pw * 32; row0 < L::kQRows; row0 += kProducerThreads) {
       // K extra: every row (1, 1, 1, 0, ...); Q extra: (-hi, -mid, -lo, 0, ...) of lse / scale
       const uint32_t one = kFp16 ? 0x3C00u : 0x3F80u;
       uint8_t* xt = smem + L::kX;
@@ -262,7 +275,9 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       uint4 kv0 = make_uint4(one | (one << 16), one, 0, 0);
       float x = 3.0e38f;                                 // padding rows: exp(-huge) = 0
       if (kFp16) x = 60000.f;
-      if (r < rows_valid) x = p.lse[(size_t)bh * p.Lq + row_base + r] * p.inv_scale;
+      const int m = m0 + (r >> 7), rr = r & 127, q_row0 = m * p.group_rows;
+      const int rows_valid = rows_of(m);
+      if (rr < rows_valid) x = p.lse[(size_t)bh * p.Lq + q_row0 + rr] * p.inv_scale;
       uint32_t w0, w1;
       if (kFp16) {
         const __half hi = __float2half_rn(x);
@@ -286,8 +301,8 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       *reinterpret_cast<uint4*>(xt + swz(r, 3)) = make_uint4(0, 0, 0, 0);
       // Q rows (through the permutation if given)
       int src = -1;
-      if (r < rows_valid) {
-        src = row_base + r;
+      if (rr < rows_valid) {
+        src = q_row0 + rr;
         if (p.perm != nullptr) src = static_cast<int>(p.perm[(size_t)bh * p.Lq + src]);
       }
       const uint8_t* qb = reinterpret_cast<const uint8_t*>(p.q) + 2 * ((size_t)b * p.q_stride[0] + (size_t)h * p.q_stride[2]) + cch * 16;
@@ -296,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       for (int i = 0; i < 32 / kRowsPerInstr; ++i) {
         const int rl = i * kRowsPerInstr + sub;
         const int id = __shfl_sync(0xffffffffu, src, rl);
-        const uint32_t dst = s_base + L::kQ + swz(row0 + rl, cch);
+        const uint32_t dst = s_base + L::kQ + swz<L::kQRows>(row0 + rl, cch);
         if (c_in_tile) {
           if (id >= 0 && c_live) cp_async16(dst, qb + (size_t)id * q_row);
           else cp_async16_zfill(dst, p.q, 0);
@@ -326,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
           if (!ok) break;
           if (tma_leader) {
             mbar_arrive_expect_tx(bar(BAR_FULL + slot), L::kTileBytes);
-            co[kmap.pos_row] = t * kTile;
+            co[kmap.pos_row] = (tile0 + t) * kTile;
 #pragma unroll
             for (int cb = 0; cb < L::kBlocks; ++cb)
               tma_load_4d(sRing(slot) + cb * 16384, kmap.k, cb * 64, co[1], co[2], co[3], bar(BAR_FULL + slot));
@@ -344,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
 #pragma unroll 4
       for (int i = pw; i < 128 / kRowsPerInstr; i += kProducerWarps) {
         const int rl = i * kRowsPerInstr + sub;
-        const int krow = t * kTile + rl;
+        const int krow = (tile0 + t) * kTile + rl;
         const uint32_t dst = dst0 + swz(rl, cch);
         if (c_in_tile) {
           if (krow < p.Lk && c_live) cp_async16(dst, kb + (size_t)krow * k_row);
@@ -364,23 +379,49 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
   }
 }
 
-template <int D, bool kFp16, int kPoly = 2>
-int launch(const GroupMassParams& p, cudaStream_t stream) {
-  using L = Smem<D>;
-  auto kern = group_mass_kernel<D, kFp16, kPoly>;
+template <int D, bool kFp16, int G = 1>
+int launch(const GroupMassParams& p, cudaStream_t stream, int splits = 1) {
+  using L = Smem<D, G>;
+  auto kern = group_mass_kernel<D, kFp16, G>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic) != cudaSuccess) return -8;
-  const long long grid = (long long)p.B * p.H * p.M;
+  const long long grid = (long long)p.B * p.H * ((p.M + G - 1) / G) * splits;
   KeyTileMap kmap{};
   // (the map carries the true head dimension: boxes that reach beyond it are zero-filled by the copy engine)
   kmap.valid = encode_tile_map(p.k, p.k_stride, p.B, p.Lk, p.H, p.D, kmap.k, kmap.pos_h, kmap.pos_row, kmap.pos_b);
-  kern<<<(unsigned)grid, kThreads, L::kDynamic, stream>>>(p, kmap);
+  kern<<<(unsigned)grid, kThreads, L::kDynamic, stream>>>(p, kmap, splits);
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
+}
+
+// Two groups per CTA (D = 128): one 128 x 256 product per key tile reads the keys once for both groups, where two 128 x 128
+// products read both operands from shared memory at its full rate: 6,516 -> 6,125 us at 24 heads x 32,760, 556 -> 535 at
+// 8 x 16,380.  But the items are twice as large: 24 heads x 4,680 (888 groups, six full waves) 178 -> 200 us.  Rows of the
+// result do not depend on one another, so the key tiles of a pair may go to several CTAs.  Returns the number of CTAs per
+// pair, or 0 for one group per CTA, by the length of the launch in key tiles of one group: a CTA's start (barriers, tensor
+// memory, its query rows) is about four, a tile of two groups 1.9.  (At D = 64 the products are half as long: 96 us against
+// 110 at 12 heads x 4,700; beside the wider tiles two groups do not fit.)
+int pair_splits(const GroupMassParams& p) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long bh = (long long)p.B * p.H, tiles = ((long long)p.Lk + kTile - 1) / kTile;
+  auto waves = [&](long long ctas) { return (double)((ctas + sms - 1) / sms); };
+  double best = waves(bh * p.M) * ((double)tiles + 4.0);
+  int splits = 0;
+  for (int s = 1; s <= 8 && s <= tiles; ++s) {
+    const long long ctas = bh * ((p.M + 1) / 2) * s;
+    const double cost = waves(ctas) * ((double)((tiles + s - 1) / s) * 1.9 + 4.0);
+    if (cost < best && ctas <= 0x7fffffffLL) { best = cost; splits = s; }
+  }
+  return splits;
 }
 
 }  // namespace
 
 int launch_group_mass(const GroupMassParams& p, bool fp16, cudaStream_t stream) {
-  if (p.D == 128) return fp16 ? launch<128, true>(p, stream) : launch<128, false>(p, stream);
+  if (p.D == 128) {
+    const int splits = pair_splits(p);
+    if (splits > 0) return fp16 ? launch<128, true, 2>(p, stream, splits) : launch<128, false, 2>(p, stream, splits);
+    return fp16 ? launch<128, true>(p, stream) : launch<128, false>(p, stream);
+  }
   if (p.D == 64) return fp16 ? launch<64, true>(p, stream) : launch<64, false>(p, stream);
   // every other multiple of 8 up to 256 (the reference's head-dimension table has 96, 144, 160, 192, 256): padded layouts
   if (p.D < 8 || p.D > 256 || p.D % 8 != 0) return -3;

@@ -123,3 +123,26 @@ def test_mass_other_head_dims(cuda_device, D):
     out1 = group_mass(q.to(dev), kd, lse1.to(dev)).cpu().double()
     assert (out1 - ref1).abs().max() / ref1.abs().max() < 2e-3
     assert torch.equal(out1, group_mass(q.to(dev), kd.contiguous(), lse1.to(dev)).cpu().double())
+
+
+# two groups per CTA (D = 128): odd numbers of groups, short groups, key stretches of unequal length
+@pytest.mark.parametrize("B,H,Lq,Lk,rows", [(1, 12, 3400, 2000, 128), (1, 40, 1200, 1100, 128), (2, 9, 2000, 900, 64), (1, 1, 130, 5000, 128),
+                                            (1, 148, 300, 130, 128)])
+def test_two_groups_per_cta(cuda_device, B, H, Lq, Lk, rows):
+    from mcsparse_b200.kernels.flash_mcsa.token_sparse import group_mass
+    g = torch.Generator().manual_seed(Lq + Lk)
+    q = torch.randn(B, H, Lq, 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    k = torch.randn(B, H, Lk, 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    perm = torch.stack([torch.randperm(Lq, generator=g) for _ in range(B * H)]).to(cuda_device)
+    idx = perm.view(B, H, Lq, 1)
+    s = torch.matmul(q.float().gather(2, idx.expand(B, H, Lq, 128)), k.float().transpose(-1, -2)) / 128 ** 0.5
+    lse = torch.logsumexp(s, -1)
+    got = group_mass(q, k, lse, group_rows=rows, perm=perm, normalize=True)
+    p = (s - lse.unsqueeze(-1)).exp()
+    for m in range(got.shape[2]):
+        want = p[:, :, m * rows:(m + 1) * rows].mean(2)
+        err = (got[:, :, m] - want).abs() / want.abs().clamp_min(1e-7)
+        assert float(err.max()) < 2e-3, (m, float(err.max()))          # the tolerance of the tests above
+    # the first group alone (one group per CTA): the same bits
+    q0 = q.gather(2, idx[:, :, :rows].expand(B, H, min(rows, Lq), 128))
+    assert torch.equal(group_mass(q0, k, lse[:, :, :rows], group_rows=rows, normalize=True)[:, :, 0], got[:, :, 0])

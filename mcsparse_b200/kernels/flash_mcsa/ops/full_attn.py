@@ -2,7 +2,7 @@
 
 Mirrors the reference's ``mcsparse/kernels/flash_mcsa/ops/full_attn.py`` (``full_attention`` :65-86,
 ``full_attention_with_lse`` :88-121).  The reference calls FlashAttention-3 (a Hopper build) and needs three
-layout copies in and one out; here both functions run this package's own attention kernel in dense mode
+layout copies in and one out; here both functions run this package's own dense attention kernel
 (``mcs_dense_attn_fwd``: every query group attends to all keys) on strided views, so there is no copy, no
 external library and no backend to resolve.  The LSE is the natural logarithm of the row sums of
 ``exp(scale * q . k)``, i.e. it includes the attention scale, as the token-probability kernel expects.
@@ -27,7 +27,7 @@ def resolve_impl(requested: str = "auto") -> str:
 
 
 def describe(resolved: str) -> str:
-    return "full attention = mcsparse_b200 dense mode of the gather-KV kernel (sm_100a)"
+    return "full attention = mcsparse_b200 dense attention kernel (sm_100a)"
 
 
 def _dense(q: Tensor, k: Tensor, v: Tensor, scale: Optional[float], want_lse: bool,

@@ -560,7 +560,8 @@ int launch_topk_select(const TopkParams& p, cudaStream_t stream) {
     if ((all || r_s < kSample) && smem <= kStreamSmemLimit) {
       const bool three = smem <= kStreamSmemLimit / 3;
       auto kern = three ? topk_stream_kernel<3, 2> : topk_stream_kernel<2, 4>;
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -8;
+      // (the limit, not this launch's size: another thread may launch the same kernel with another size in between)
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmemLimit) != cudaSuccess) return -8;
       const long long slots = (long long)(three ? 3 : smem <= kStreamSmemLimit / 2 ? 2 : 1) * sms;
       kern<<<(unsigned)(p.rows < slots ? p.rows : slots), kST, smem, stream>>>(p, (int)cap, words);
       return cudaGetLastError() == cudaSuccess ? 0 : -8;
@@ -571,7 +572,8 @@ int launch_topk_select(const TopkParams& p, cudaStream_t stream) {
   const size_t smem = sizeof(Shared) + (stage ? row_bytes : 0);
   const int grid = (int)(p.rows < (long long)sms ? p.rows : sms);
   if (stage) {
-    if (cudaFuncSetAttribute(topk_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -8;
+    if (cudaFuncSetAttribute(topk_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(Shared) + topk_stage_limit_bytes())) != cudaSuccess)
+      return -8;
     topk_select_kernel<true><<<grid, kThreads, smem, stream>>>(p);
   } else {
     topk_select_kernel<false><<<grid, kThreads, smem, stream>>>(p);

@@ -107,3 +107,32 @@ def test_streaming_edges(cuda_device, L, k_total):
     shifted = torch.empty(scores.numel() + 1, device=cuda_device)[1:].view(scores.shape)   # 4-byte aligned base
     shifted.copy_(scores)
     assert torch.equal(_run(cuda_device, shifted, k_total, ranges), ref)
+
+
+def test_threads_with_different_row_lengths(cuda_device):
+    """Launches of one kernel with different shared-memory sizes from several threads at once."""
+    import threading
+    from mcsparse_b200.kernels.flash_mcsa.token_sparse import select_topk_with_sinks
+    shapes = [(4100, 512), (98280, 4096), (32760, 2048), (32760, 12000), (49000, 40000), (8200, 100)]
+    data = []
+    for L, k in shapes:
+        s = torch.rand(40, L, generator=torch.Generator().manual_seed(L + k)) ** 8
+        data.append((s.to(cuda_device), k, select_topk_ref(s, k, sinks=range(4))))
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(i):
+        try:
+            with torch.cuda.device(cuda_device), torch.cuda.stream(torch.cuda.Stream()):
+                for n in range(30):
+                    s, k, ref = data[(i + n) % len(data)]
+                    out = select_topk_with_sinks(s, k, [(0, 4)])
+                    if n >= 24 and not torch.equal(out.cpu(), ref):
+                        errors.append((i, n))
+        except Exception as e:                               # noqa: BLE001 (reported below)
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors, errors

@@ -59,10 +59,12 @@ def test_dense_argument_errors(cuda_device):
 # edges of the two-stream kernel: one row, one key, stream B empty / one row, several items per CTA; and layouts that no
 # tensor map describes (keys shared by all heads: stride 0), which take the gathering kernel
 @pytest.mark.parametrize("Lq,Lk,D,shared", [(1, 1, 128, False), (128, 129, 64, False), (129, 127, 128, False), (256, 640, 64, False),
-                                            (513, 300, 128, False), (5000, 200, 64, False), (300, 260, 128, True), (257, 130, 64, True)])
+                                            (513, 300, 128, False), (5000, 200, 64, False), (300, 260, 128, True), (257, 130, 64, True),
+                                            (5000, 129, 128, False), (1025, 260, 128, False), (1153, 1, 64, False)])
 def test_dense_edges(cuda_device, Lq, Lk, D, shared):
     from mcsparse_b200.kernels.flash_mcsa.ops.full_attn import full_attention_with_lse
-    B, H = (1, 18) if Lq == 5000 else (2, 3)
+    # (more groups of 128 rows than SMs: the dense kernel; fewer: the gathering one)
+    B, H = (1, 18) if Lq >= 1025 else (2, 3)
     g = torch.Generator().manual_seed(Lq + Lk)
     q = torch.randn(B, H, Lq, D, generator=g).to(torch.bfloat16)
     k = (torch.randn(B, 1 if shared else H, Lk, D, generator=g) * torch.linspace(0.2, 3.0, Lk).view(1, 1, Lk, 1)).to(torch.bfloat16)

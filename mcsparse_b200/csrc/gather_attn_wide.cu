@@ -12,7 +12,8 @@
 // (batch, head)), 13 warps:
 //   warps 0-7   softmax and epilogue: thread == query row == tensor-memory lane, warps w and w + 4 share their rows and take
 //               the column halves 0-63 and 64-127 of every tile; they agree on one running maximum by a two-warp
-//               barrier-with-OR per tile, as in the main kernel
+//               barrier-with-OR per tile, as in the main kernel (e4m3: a second barrier hands the lower half's row sums to the
+//               upper half)
 //   warps 8-11  producers: 16-byte cp.async row gathers of Q, then K(0), K(1), V(0), K(2), V(1), ... into a ring
 //               of 2-5 tile slots
 //   warp 12     issues S = Q K^T (SS) and O += P V (P from tensor memory, V as an MN-major operand) in the order
@@ -23,7 +24,8 @@
 // What bounds it: the softmax of a tile (two warps per sub-partition) and the row gather, 256 rows of 2 D bytes per tile.
 // With four softmax warps over whole rows and one score buffer a tile took 4,900 cycles at every head dimension.
 // Measured (8 heads x 20,475 tokens, 3,072 selected, permutation and residual): D = 144 fp16 580 -> 471 us (290 GFLOP;
-// 176 us at the measured burst rate), 96 418 -> 371, 160 574 -> 522, 192 581 -> 556, 256 687 -> 664, e4m3 160 435 -> 389.
+// 176 us at the measured burst rate), 96 418 -> 371, 160 574 -> 522, 192 581 -> 556, 256 687 -> 664, e4m3 160 395 -> 354
+// (the rule by whole rows costs 2 us of it).
 // Every mbarrier wait is bounded and reports through the status
 // word; a role whose wait expires leaves its loop, the others follow through their own bounded waits.
 #include <cuda_bf16.h>
@@ -63,8 +65,9 @@ struct SmemW {
   static constexpr int kRingOff = kTileBytes;
   static constexpr int kBars = kRingOff + kRing * kTileBytes;
   static constexpr int kXch = kBars + WB_COUNT * 8;            // float [2 halves][128]: tile maxima, exchanged on a raise
-  static constexpr int kFlag = kXch + 1024;                    // float [2][128]: dominant-maximum flags (e4m3)
-  static constexpr int kSum = kFlag + 1024;                     // float [2][128]: row sums
+  static constexpr int kChain = kXch + 1024;                   // float4 [128]: the four running sums of the lower half (e4m3)
+  static constexpr int kRow = kChain + 2048;                   // float [128]: the row's sum so far, exchanged with the maxima (e4m3)
+  static constexpr int kSum = kRow + 512;                      // float [2][128]: row sums
   static constexpr int kTmemSlot = kSum + 1024;
   static constexpr int kTotal = kTmemSlot + 16;
   static constexpr int kDynamic = kTotal + 1024;
@@ -171,9 +174,11 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
     const int x = warp >> 2;                            // column half
     const int r_in = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = (static_cast<uint32_t>(warp & 3) * 32u) << 16;
-    const int pair_bar = 1 + (warp & 3);                // named barrier of this row block's two warps
+    const int pair_bar = 1 + (warp & 3);                // named barriers of this row block's two warps
+    const int sum_bar = 5 + (warp & 3);                 // (e4m3: from the lower half to the upper)
     float* xch = reinterpret_cast<float*>(smem + L::kXch);
-    float* flag = reinterpret_cast<float*>(smem + L::kFlag);
+    float4* chain = reinterpret_cast<float4*>(smem + L::kChain);
+    float* row_sum = reinterpret_cast<float*>(smem + L::kRow);
     const float scale_log2 = kFp8 ? p.scale_qk_log2[item] : p.scale_log2;
     const unsigned long long scale2 = f2_pack(scale_log2, scale_log2);
     // lazy raise of the running maximum with the thresholds of the main kernel; e4m3 P is biased by 2^4 so that the
@@ -184,7 +189,9 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
     const int half_chunks = (n_pv / 8 + 1) / 2;
     const int c_lo = x * half_chunks, c_hi = x == 0 ? half_chunks : n_pv / 8;
     const uint32_t tO = tmem + kColOW + lane_addr;
-    float m_run = -INFINITY, l_run = 0.f;               // running maximum (the same in both halves), this half's row sum
+    // running maximum (the same in both halves); row sum of this half, for e4m3 that of the whole row (upper half) or a bound
+    // below it (lower half: the whole row's at the last exchange, its own half's since)
+    float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     int fail_g = 0;
     bool fail_bar_done = false;
@@ -213,24 +220,27 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
 #pragma unroll
         for (int q = 0; q < 4; ++q) mx[q] = fmax3(mx[q], __uint_as_float(sc[i + 2 * q]), __uint_as_float(sc[i + 2 * q + 1]));
       const float m_loc = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]) * scale_log2;
-      bool want = (m_loc - m_run) > kRescale, dom = false;
-      if constexpr (kFp8) {
-        // a new maximum that would hold more than an eighth of the mass so far becomes the reference point at once:
-        // its e4m3 probability is then exact (see the main kernel)
-        dom = (m_loc > m_run) && (ex2_approx(m_loc - m_run + kBias) > 0.125f * l_run);
-        want = want || dom;
-      }
+      float alpha = 1.f;
+      bool want = (m_loc - m_run) > kRescale;
+      // e4m3: a new maximum that would hold more than an eighth of the row's mass so far becomes the reference point at once:
+      // its probability is then exact (see the main kernel).  The rule goes by the mass of the whole row: by the mass of a half
+      // the reference would move sooner and round every probability behind it at another scale.  The upper half's thread has
+      // that mass, the lower half's a bound below it (with a margin for the rounding of its sums) and so may want an exchange
+      // that then raises nothing.
+      if constexpr (kFp8) want = want || ((m_loc > m_run) && (ex2_approx(m_loc - m_run + kBias) > (x == 0 ? 0.124f : 0.125f) * l_run));
       if (named_bar_red_or(pair_bar, 64, want)) {
         xch[x * 128 + r_in] = m_loc;
-        if constexpr (kFp8) flag[x * 128 + r_in] = dom ? 1.f : 0.f;
+        if (kFp8 && x == 1) row_sum[r_in] = l_run;
         named_bar_sync(pair_bar, 64);
         const float m_new = fmaxf(m_loc, xch[(x ^ 1) * 128 + r_in]);
         bool raise = (m_new - m_run) > kRescale;            // the same decision in both threads of the row
-        if constexpr (kFp8) raise = raise || ((dom || flag[(x ^ 1) * 128 + r_in] != 0.f) && m_new > m_run);
-        const float alpha = raise ? ex2_approx(m_run - m_new) : 1.f;
-        if (raise) m_run = m_new;
-        l_run *= alpha;
-        if (g > 0) {
+        if constexpr (kFp8) {
+          if (x == 0) l_run = row_sum[r_in];
+          raise = raise || ((m_new > m_run) && (ex2_approx(m_new - m_run + kBias) > 0.125f * l_run));
+        }
+        if (raise) { alpha = ex2_approx(m_run - m_new); m_run = m_new; }
+        if (!kFp8 || x == 0) l_run *= alpha;
+        if (g > 0 && (!kFp8 || __any_sync(0xffffffffu, raise))) {
           // O is stable once P V of the previous tile has completed (this tile's P V waits for the stores below)
           ok = mbar_wait(bar(WB_PV_DONE), (g - 1) & 1, p.status, 61);
           if (!ok) { fail_g = g; fail_bar_done = true; break; }
@@ -249,7 +259,7 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
       }
       const float neg_m = kBias - m_run;
       const unsigned long long neg2 = f2_pack(neg_m, neg_m);
-      unsigned long long ls[2] = {0ull, 0ull};
+      unsigned long long ls[2] = {0ull, 0ull};             // e4m3: four sums, over the columns of each residue modulo 4
 #pragma unroll
       for (int c = 0; c < (kFp8 ? 2 : 4); ++c) {
         uint32_t pk[8];
@@ -262,6 +272,7 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
             const float p0 = ex2_approx(ya.x), p1 = ex2_approx(ya.y), p2 = ex2_approx(yb.x), p3 = ex2_approx(yb.y);
             ls[0] = f2_add(ls[0], f2_pack(p0, p1));
             ls[1] = f2_add(ls[1], f2_pack(p2, p3));
+            sc[e] = __float_as_uint(p0); sc[e + 1] = __float_as_uint(p1); sc[e + 2] = __float_as_uint(p2); sc[e + 3] = __float_as_uint(p3);
             pk[i] = pack_e4m3x4(p0, p1, p2, p3);
           } else {
             const int e = c * 16 + 2 * i;
@@ -274,10 +285,30 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
         tmem_st8(tS + c * 8, pk);
       }
       const float2 l0 = f2_unpack(ls[0]), l1 = f2_unpack(ls[1]);
-      l_run += (l0.x + l0.y) + (l1.x + l1.y);
+      if (!kFp8 || x == 0) l_run += (l0.x + l0.y) + (l1.x + l1.y);
+      if (kFp8 && x == 0) chain[r_in] = make_float4(l0.x, l0.y, l1.x, l1.y);
       tmem_wait_st();
       tc_fence_before();
       warp_arrive(bar(WB_P_READY + buf));
+      if constexpr (kFp8) {
+        // The upper half continues the four sums of the lower half in the order of the columns, so that the row's sum, and with
+        // it the rule above, does not depend on how the row is split.  This runs under the tile's P V.  (The lower half only
+        // announces its sums; it overwrites them behind the next tile's barrier.)
+        if (x == 0) {
+          named_bar_arrive(sum_bar, 64);
+        } else {
+          named_bar_sync(sum_bar, 64);
+          const float4 s = chain[r_in];
+          unsigned long long sa = f2_pack(s.x, s.y), sb = f2_pack(s.z, s.w);
+#pragma unroll
+          for (int i = 0; i < 64; i += 4) {
+            sa = f2_add(sa, f2_pack(__uint_as_float(sc[i]), __uint_as_float(sc[i + 1])));
+            sb = f2_add(sb, f2_pack(__uint_as_float(sc[i + 2]), __uint_as_float(sc[i + 3])));
+          }
+          const float2 a = f2_unpack(sa), c = f2_unpack(sb);
+          l_run = l_run * alpha + ((a.x + a.y) + (c.x + c.y));
+        }
+      }
     }
     if (!ok) {
       // failure path: a bounded wait expired (the status word says where).  The partner warp may still be running; a named
@@ -286,11 +317,14 @@ __global__ void __launch_bounds__(kThreadsW, 1) gather_attn_wide_kernel(const Ga
       for (int g = fail_g; g < T; ++g) {
         if (!done && named_bar_red_or(pair_bar, 64, false)) named_bar_sync(pair_bar, 64);
         done = false;
+        if constexpr (kFp8) {
+          if (x == 0) named_bar_arrive(sum_bar, 64); else named_bar_sync(sum_bar, 64);
+        }
       }
     }
-    // ---- the row's sum: both halves, relative to the same maximum
+    // ---- the row's sum: both halves, relative to the same maximum (e4m3: the upper half's thread has it all)
     float* sums = reinterpret_cast<float*>(smem + L::kSum);
-    sums[x * 128 + r_in] = l_run;
+    sums[x * 128 + r_in] = kFp8 && x == 0 ? 0.f : l_run;
     ok = !named_bar_red_or(pair_bar, 64, !ok);
     const float l_all = sums[r_in] + sums[128 + r_in];
     if (ok) ok = mbar_wait(bar(WB_O_FULL), 0, p.status, 62);

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "pddp_key.cuh"
 #include "ptx.cuh"
 
 namespace mcs {
@@ -252,7 +253,7 @@ __device__ __forceinline__ void project_rows(uint32_t s_base, int warp, int lane
     const float a = project_row<D, kFp16>(s_base + buf * kTileBytes, mine, vec);
     const int r = t * 128 + mine;
     if (r < rows) {
-      keys[r_first + r] = ((unsigned long long)float_key(a) << 32) | (unsigned)(r_first + r);
+      keys[r_first + r] = sort_key(float_key(a), r_first + r);
       if (proj_out != nullptr) proj_out[r] = a;
     }
     __syncwarp();
@@ -426,9 +427,13 @@ __global__ void __launch_bounds__(kNodeThreads, 2) pddp_node_kernel(PddpParams p
         unsigned long long* keys = p.keys + (size_t)bh * p.key_stride + (size_t)node * pad;
         project_rows<D, kFp16>(s_base, warp, lane, xb, row_bytes, ids, rows, 0, vec, keys,
                                proj_out != nullptr ? proj_out + (size_t)bh * p.N + pos0 : nullptr, n_tiles <= kBufs);
-        for (int r = rows + tid; r < pad; r += 128) keys[r] = 0xFFFFFFFFFFFFFFFFull;
+        for (int r = rows + tid; r < pad; r += 128) keys[r] = kPadKey;
         cp_async_wait_all();
       }
+    } else if (size <= kChunkRows) {
+      // a wait expired (the status word says where): the node keeps its order, so that the sort finds a key in every slot
+      unsigned long long* keys = p.keys + (size_t)bh * p.key_stride + (size_t)node * pad;
+      for (int r = tid; r < pad; r += 128) keys[r] = r < rows ? sort_key(0u, r) : kPadKey;
     }
     tc_fence_before();
   } else {
@@ -559,7 +564,7 @@ __global__ void __launch_bounds__(128) pddp_project_kernel(PddpParams p, int lv,
                          2 * (size_t)p.x_stride_row, perm_in + (size_t)bh * p.N + pos0, rows, row_begin, vec, keys,
                          proj_out != nullptr ? proj_out + (size_t)bh * p.N + pos0 : nullptr, false);
   if (row_begin + rows == size)
-    for (int r = size + tid; r < pad; r += 128) keys[r] = 0xFFFFFFFFFFFFFFFFull;           // slots beyond the node sort last
+    for (int r = size + tid; r < pad; r += 128) keys[r] = kPadKey;             // slots beyond the node sort last
   cp_async_wait_all();
 }
 
@@ -737,9 +742,9 @@ __global__ void __launch_bounds__(256) pddp_wide_project_kernel(PddpParams p, in
     if (lane == 0) {
       const int r = r0 + i;
       if (r >= nsize) {
-        keys[slot0 + i] = 0xFFFFFFFFFFFFFFFFull;
+        keys[slot0 + i] = kPadKey;
       } else {
-        keys[slot0 + i] = ((unsigned long long)float_key(acc) << 32) | (unsigned)r;
+        keys[slot0 + i] = sort_key(float_key(acc), r);
         if (proj_out != nullptr) proj_out[(size_t)bh * p.N + pos0 + i] = acc;
       }
     }
@@ -778,7 +783,7 @@ __global__ void __launch_bounds__(kT) pddp_sort_kernel(PddpParams p, int lv, lon
     for (int i = 0; i < 4; ++i) { const ulonglong2 v = src[i]; a[2 * i] = v.x; a[2 * i + 1] = v.y; }
   } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a[i] = 0xFFFFFFFFFFFFFFFFull;
+    for (int i = 0; i < 8; ++i) a[i] = kPadKey;
   }
   auto cmpx = [&](int i, int j, bool asc) {
     const bool swap = (a[i] > a[j]) == asc;
@@ -833,7 +838,7 @@ __global__ void __launch_bounds__(kT) pddp_sort_kernel(PddpParams p, int lv, lon
     const size_t start = (size_t)blockIdx.y * p.N + T.node_start[node];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (gi + i < size) perm_out[start + gi + i] = perm_in[start + (size_t)(a[i] & 0xFFFFFFFFull)];
+      if (gi + i < size) perm_out[start + gi + i] = perm_in[start + key_position(a[i], size)];
   } else {
     ulonglong2* dst = reinterpret_cast<ulonglong2*>(keys + slot0);
 #pragma unroll

@@ -60,8 +60,10 @@ def pddp_start_vectors(BH: int, N: int, C: int, D: int, seed: int = 0) -> Tensor
 class _StartVectorPool:
     """Device copies of the default start vectors, which depend on nothing but (BH, N, C, D, seed): a denoising run groups
     the queries of every layer with the same ones.  Drawing them takes the host 3.4 ms at 24 heads x 32,760 tokens, the
-    grouping itself 1.4 ms.  Bounded (least recently used entries go first), shared by all threads, and every use is
-    recorded on the stream that reads the tensor, so an entry that is dropped stays valid until its readers are done."""
+    grouping itself 1.2 ms.  Bounded (least recently used entries go first), shared by all threads, and every use is
+    recorded on the stream that reads the tensor, so an entry that is dropped stays valid until its readers are done.
+    That does not reach the replays of a captured graph, which would keep the bare address: an entry is refused while the
+    stream is being captured, whether it is there already or not."""
 
     MAX_ENTRIES, MAX_BYTES = 16, 64 << 20
 
@@ -70,6 +72,10 @@ class _StartVectorPool:
         self._entries = OrderedDict()
 
     def get(self, BH: int, N: int, C: int, D: int, seed: int, device) -> Tensor:
+        with torch.cuda.device(device):
+            if torch.cuda.is_current_stream_capturing():
+                raise RuntimeError("the default start vectors cannot be used in a graph capture: pass start_vectors "
+                                   "(pddp_start_vectors(...), on the device) and keep them as long as the graph")
         key = (device.index if device.index is not None else torch.cuda.current_device(), BH, N, C, D, seed)
         with self._lock:
             sv = self._entries.get(key)
@@ -96,7 +102,7 @@ _start_vectors = _StartVectorPool()
 
 
 def release_start_vectors() -> None:
-    """Give back the device memory of the start vectors kept between calls."""
+    """Give back the device memory of the start vectors kept between calls (no captured graph reads them)."""
     _start_vectors.clear()
 
 
@@ -109,7 +115,8 @@ def pca_group_perm(x: Tensor, C: int = 128, pow_iters: int = 4, seed: int = 0, p
     (64 and 128 on the tensor-core Gram path, the others on Gram-free power iterations).
     Returns perm (BH, N) int64: ``x[b, perm[b, i]]`` is the i-th reordered token.  ``proj_dim`` (an
     option the reference leaves off by default) is not part of this path.  ``return_debug`` adds the
-    per-level fp32 projections (levels, BH, N) and orders (levels + 1, BH, N).
+    per-level fp32 projections (levels, BH, N) and orders (levels + 1, BH, N).  Inside a CUDA graph capture
+    ``start_vectors`` have to be given, fp32 on x's device, and kept by the caller as long as the graph.
     """
     if proj_dim is not None:
         raise NotImplementedError("proj_dim is not part of the accelerated path")

@@ -191,7 +191,10 @@ __device__ __forceinline__ Item decode_item(const GatherAttnParams& p, int item)
 // as it lies in memory (MN-major MMA operand), so neither the Hopper kernel's in-smem transpose nor
 // its d-column pre-permutation exists here.
 template <int D, int kType, bool kDense>
-__global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAttnParams p) {
+__global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAttnParams p,
+                                                                    const __grid_constant__ DenseTileMaps maps) {
+  // dense mode with valid tensor maps: K/V tiles arrive by TMA (one elected thread, two 16 KB boxes per tile)
+  const bool use_tma = kDense && maps.valid != 0;
   constexpr bool kFp16 = kType == 1;
   constexpr bool kFp8 = kType == 2;
   constexpr int kEs = kFp8 ? 1 : 2;              // bytes per Q/K/V element
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAt
   // ---- setup
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) {
-      mbar_init(bar(BAR_FULL + i), kProducerThreads);
+      mbar_init(bar(BAR_FULL + i), use_tma ? 1 : kProducerThreads);
       mbar_init(bar(BAR_EMPTY + i), 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -447,7 +450,8 @@ __global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAt
     //
     // Producer warp pw gathers tile rows 32*pw..+31 of every K, V and Q tile with 16-byte cp.async (the
     // softmax warps never use the load/store unit, so they are never queued behind the hundreds of copies
-    // in flight).
+    // in flight).  In the dense mode with tensor maps one elected thread of warp 0 issues the K/V tiles as
+    // TMA boxes instead and the four warps only gather Q.
     // =====================================================================
     const int pw = warp - kProducerWarp0;
     const int row0 = pw * kRowsPerProducerWarp;
@@ -498,6 +502,27 @@ __global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAt
       size_t ioff;           // the same as an offset into the index tensor (packed form)
       const uint8_t* kv;     // K or V base of (b, h) + chunk offset of this lane
     };
+    const bool tma_leader = elect_one();
+    auto load_tile_tma = [&](const Cur& c, bool is_v) {
+      // dense mode: the tile is 128 consecutive key rows of one (batch, head): kBlocks TMA boxes of 128 rows x
+      // 128 bytes, issued by one thread of producer warp 0; rows beyond the sequence end arrive as zeros
+      if (pw == 0) {
+        if (wrapped) ok = ok && mbar_wait(bar(BAR_EMPTY + slot), slot_phase ^ 1, p.status, 20);
+        if (!ok) return;
+        if (tma_leader) {
+          mbar_arrive_expect_tx(bar(BAR_FULL + slot), L::kTileBytes);
+          const void* map = is_v ? static_cast<const void*>(maps.v) : static_cast<const void*>(maps.k);
+          int co[4] = {0, 0, 0, 0};
+          co[is_v ? maps.v_pos_h : maps.k_pos_h] = c.h;
+          co[is_v ? maps.v_pos_row : maps.k_pos_row] = c.t * kTileN;
+          co[is_v ? maps.v_pos_b : maps.k_pos_b] = c.b;
+#pragma unroll
+          for (int cb = 0; cb < L::kBlocks; ++cb)
+            tma_load_4d(sRing(slot) + cb * 16384, map, cb * (128 / kEs), co[1], co[2], co[3], bar(BAR_FULL + slot));
+        }
+      }
+      if (++slot == kRing) { slot = 0; slot_phase ^= 1; wrapped = true; }
+    };
     auto load_tile = [&](const uint8_t* lane_src, size_t row_bytes, int idx, bool is_v) {
       if (wrapped) ok = ok && mbar_wait(bar(BAR_EMPTY + slot), slot_phase ^ 1, p.status, 20);
       if (!ok) return;
@@ -538,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAt
       set_item(vc, p.v, p.v_stride);
       enter_item(kc.item, kc.ic);
       int idx_k = load_idx(kc);
-      load_tile(kc.kv, k_row, idx_k, false);
+      if (use_tma) load_tile_tma(kc, false); else load_tile(kc.kv, k_row, idx_k, false);
       int idx_v = idx_k;
       auto advance_k = [&]() {
         if (++kc.t >= kc.T) {
@@ -558,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAt
         if (had_k) {
           if (kc.t == 0) enter_item(kc.item, kc.ic);
           if (!ok) break;
-          load_tile(kc.kv, k_row, idx_cur, false);
+          if (use_tma) load_tile_tma(kc, false); else load_tile(kc.kv, k_row, idx_cur, false);
           if (!ok) break;
           advance_k();
           have_k = kc.item < n_items;
@@ -568,7 +593,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_attn_kernel(const GatherAt
           // no K entry in this (final) step: skip its ring number so that V(g) is always entry 2g+2
           if (++slot == kRing) { slot = 0; slot_phase ^= 1; wrapped = true; }
         }
-        load_tile(vc.kv, v_row, idx_v, true);
+        if (use_tma) load_tile_tma(vc, true); else load_tile(vc.kv, v_row, idx_v, true);
         if (!ok) break;
         idx_v = idx_cur;                           // V(g+1) uses the indices of K(g+1)
         if (++vc.t >= vc.T) {
@@ -921,14 +946,14 @@ int num_sms() {
 }
 
 template <int D, int kType, bool kDense = false>
-int launch(const GatherAttnParams& p, cudaStream_t stream) {
+int launch(const GatherAttnParams& p, cudaStream_t stream, const DenseTileMaps& maps = DenseTileMaps{}) {
   using L = Smem<D * (kType == 2 ? 1 : 2), kType == 2 ? 256 * D : 0>;
   auto kern = gather_attn_kernel<D, kType, kDense>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
   if (e != cudaSuccess) return -8;
   const long long items = (long long)p.B * p.H * p.M;
   const int grid = (int)(items < num_sms() ? items : num_sms());
-  kern<<<grid, kThreads, L::kDynamic, stream>>>(p);
+  kern<<<grid, kThreads, L::kDynamic, stream>>>(p, maps);
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
@@ -936,16 +961,17 @@ int launch(const GatherAttnParams& p, cudaStream_t stream) {
 
 int launch_gather_attn_16bit(const GatherAttnParams& p, bool fp16, cudaStream_t stream) {
   if (p.dense) {
-    // K and V in a layout that a tensor map describes (every call of this package): the dense kernel.  Others gather
-    // consecutive rows here, in an instantiation of its own so that the sparse kernel's inner loops carry none of it.
-    // So do launches of no more groups of 128 rows than there are SMs: with one group per SM the two streams of the dense
-    // kernel would only halve the number of SMs at work (a pair of tiles takes it 3,146 cycles, one tile about 2,100 here:
-    // 56 us against 39 at a short clip with few heads).
+    // Consecutive keys: with K and V in a layout that a tensor map describes (every call of this package) their tiles come by
+    // TMA, in the dense kernel or here.  Launches of no more groups of 128 rows than there are SMs stay here, in an
+    // instantiation of its own so that the sparse kernel's inner loops carry none of it: with one group per SM the two streams
+    // of the dense kernel would only halve the number of SMs at work: 4 heads x 4,700 x 128 take 72.6 us there and 44.7 here
+    // (46.4 with the key rows copied by cp.async; 1 head x 18,900: 157 and 165 us).
     const long long groups = (long long)p.B * p.H * ((p.Sq + 127) / 128);
     DenseTileMaps maps{};
-    if ((p.D == 64 || p.D == 128) && groups > num_sms() && dense_tile_maps(p, maps)) return launch_dense_attn(p, maps, fp16, stream);
-    if (p.D == 128) return fp16 ? launch<128, 1, true>(p, stream) : launch<128, 0, true>(p, stream);
-    if (p.D == 64) return fp16 ? launch<64, 1, true>(p, stream) : launch<64, 0, true>(p, stream);
+    if (p.D == 64 || p.D == 128) dense_tile_maps(p, maps);
+    if (maps.valid && groups > num_sms()) return launch_dense_attn(p, maps, fp16, stream);
+    if (p.D == 128) return fp16 ? launch<128, 1, true>(p, stream, maps) : launch<128, 0, true>(p, stream, maps);
+    if (p.D == 64) return fp16 ? launch<64, 1, true>(p, stream, maps) : launch<64, 0, true>(p, stream, maps);
     return -3;
   }
   if (p.D == 128) return fp16 ? launch<128, 1>(p, stream) : launch<128, 0>(p, stream);

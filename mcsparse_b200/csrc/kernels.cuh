@@ -42,7 +42,7 @@ struct alignas(64) DenseTileMaps {
   unsigned long long v[16];
   int k_pos_h, k_pos_row, k_pos_b;
   int v_pos_h, v_pos_row, v_pos_b;
-  int valid;
+  int valid;     // 0: maps not built, the dense mode gathers rows with cp.async like the sparse mode
 };
 
 // (tensor_map.cu) 4-D tensor map of a (B, S, H, D) tensor of 16-bit elements with element strides {batch, row,

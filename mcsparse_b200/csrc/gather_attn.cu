@@ -957,19 +957,27 @@ int launch(const GatherAttnParams& p, cudaStream_t stream, const DenseTileMaps& 
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
+// Dense mode: whether the two-stream kernel (pairs of groups of 128 rows) ends before this one (single groups).  Both keep one
+// CTA per SM, so a launch takes its number of waves; a pair takes 1.7 times a group at D = 128 and 1.5 times at D = 64
+// (measured 1.55 to 1.77 and 1.45 to 1.5 over 4,700 to 32,760 keys).  Times in us here / there, D = 128 with 4,700 keys:
+//   heads (groups)   4 (148)     6 (222)     8 (296)     12 (444)    13 (481)    18 (666)    22 (814)
+//   waves            1 / 1       2 / 1       2 / 2       3 / 2       4 / 2       5 / 3       6 / 3
+//                    45 / 73     85 / 74     84 / 142    122 / 145   159 / 144   201 / 213   245 / 213
+bool dense_kernel_shorter(const GatherAttnParams& p) {
+  const long long heads = (long long)p.B * p.H, sms = num_sms();
+  const long long here = (heads * ((p.Sq + 127) / 128) + sms - 1) / sms, there = (heads * ((p.Sq + 255) / 256) + sms - 1) / sms;
+  return there * (p.D == 64 ? 15 : 17) < here * 10;
+}
+
 }  // namespace
 
 int launch_gather_attn_16bit(const GatherAttnParams& p, bool fp16, cudaStream_t stream) {
   if (p.dense) {
     // Consecutive keys: with K and V in a layout that a tensor map describes (every call of this package) their tiles come by
-    // TMA, in the dense kernel or here.  Launches of no more groups of 128 rows than there are SMs stay here, in an
-    // instantiation of its own so that the sparse kernel's inner loops carry none of it: with one group per SM the two streams
-    // of the dense kernel would only halve the number of SMs at work: 4 heads x 4,700 x 128 take 72.6 us there and 44.7 here
-    // (46.4 with the key rows copied by cp.async; 1 head x 18,900: 157 and 165 us).
-    const long long groups = (long long)p.B * p.H * ((p.Sq + 127) / 128);
+    // TMA, in the dense kernel or in an instantiation of this one (so that the sparse kernel's inner loops carry none of it).
     DenseTileMaps maps{};
     if (p.D == 64 || p.D == 128) dense_tile_maps(p, maps);
-    if (maps.valid && groups > num_sms()) return launch_dense_attn(p, maps, fp16, stream);
+    if (maps.valid && dense_kernel_shorter(p)) return launch_dense_attn(p, maps, fp16, stream);
     if (p.D == 128) return fp16 ? launch<128, 1, true>(p, stream, maps) : launch<128, 0, true>(p, stream, maps);
     if (p.D == 64) return fp16 ? launch<64, 1, true>(p, stream, maps) : launch<64, 0, true>(p, stream, maps);
     return -3;

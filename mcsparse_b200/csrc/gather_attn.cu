@@ -965,7 +965,7 @@ int launch(const GatherAttnParams& p, cudaStream_t stream, const DenseTileMaps& 
 //                    45 / 73     85 / 74     84 / 142    122 / 145   159 / 144   201 / 213   245 / 213
 bool dense_kernel_shorter(const GatherAttnParams& p) {
   const long long heads = (long long)p.B * p.H, sms = num_sms();
-  const long long here = (heads * ((p.Sq + 127) / 128) + sms - 1) / sms, there = (heads * ((p.Sq + 255) / 256) + sms - 1) / sms;
+  const long long here = (heads * p.M + sms - 1) / sms, there = (heads * ((p.Sq + 255) / 256) + sms - 1) / sms;
   return there * (p.D == 64 ? 15 : 17) < here * 10;
 }
 

@@ -176,17 +176,43 @@ def select_topk_var(scores: torch.Tensor, k_rows: torch.Tensor, k_max: int, sink
     return out
 
 
+def selection_counts(L_K: int, n_sink: int, tile_n: int, base_counts: torch.Tensor) -> torch.Tensor:
+    """Budget arithmetic of the variable-length modes (token_sparse.py:811-823, :902-923): the per-row number of
+    ranked tokens is rounded up to whole tiles (never beyond L_K), the sinks are added, the total is rounded up to whole
+    tiles again as long as ranked tokens are left to fill it, else down, and it is at least one tile.  Integer tensors on
+    any device; ``selection_budgets`` is the same in one launch."""
+    c = base_counts.long().clamp(min=1)
+    c = (((c + tile_n - 1) // tile_n) * tile_n).clamp(max=L_K)
+    avail = int(c.max().item()) + n_sink                      # length of [sinks, ranked prefix] in the reference
+    if n_sink:
+        c = (((c + n_sink + tile_n - 1) // tile_n) * tile_n).clamp(max=avail)
+    cap = max(tile_n, min(((L_K + tile_n - 1) // tile_n) * tile_n, (avail // tile_n) * tile_n))
+    c = c.clamp(min=tile_n, max=cap)
+    return ((c // tile_n) * tile_n).clamp(max=L_K)
+
+
+def _ranked_counts(t: torch.Tensor, L_K: int, what: str) -> torch.Tensor:
+    """Integer counts as contiguous int32 on the GPU (a count beyond the row means the whole row)."""
+    if t.dtype not in (torch.int32, torch.int64, torch.int16, torch.int8, torch.uint8):
+        raise TypeError(f"{what} must be an integer tensor, got {t.dtype}")
+    if not t.is_cuda:
+        raise RuntimeError(f"{what} must be a CUDA tensor")
+    if t.dtype == torch.int64:
+        t = t.clamp(min=0, max=L_K)
+    return t.to(torch.int32).contiguous()
+
+
 def selection_budgets(L_K: int, n_sink: int, tile_n: int, base: torch.Tensor, floor_rows: Optional[torch.Tensor] = None,
                       floor_all: int = 0):
-    """Budget arithmetic of the variable-length modes (token_sparse.py:811-823, :902-923): the per-row number of
-    ranked tokens (at least ``floor_rows`` / ``floor_all``) is rounded up to whole tiles (never beyond L_K), the sinks are
-    added, the total is rounded up to whole tiles again as long as ranked tokens are left to fill it, else down, and it
-    is at least one tile.  ``base`` and ``floor_rows``: int32 CUDA tensors, one entry per row.  Returns budgets in
-    tokens, tile counts (both int32, shape of ``base``) and the largest budget as a number (the host waits for it: it is
-    the width of the index list)."""
-    base = base.contiguous()
+    """``selection_counts`` of per-row numbers of ranked tokens, each at least ``floor_rows`` (per row) or ``floor_all``, in
+    one launch.  ``base`` and ``floor_rows``: integer CUDA tensors, one entry per row.  Returns budgets in tokens, tile
+    counts (both int32, shape of ``base``) and the largest budget as a number (the host waits for it: it is the width of
+    the index list)."""
+    base = _ranked_counts(base, L_K, "base")
     if floor_rows is not None:
-        floor_rows = floor_rows.to(torch.int32).contiguous()
+        floor_rows = _ranked_counts(floor_rows, L_K, "floor_rows")
+        if floor_rows.numel() != base.numel() or floor_rows.device != base.device:
+            raise ValueError("floor_rows must have one entry per row, on base's device")
     budgets, tiles = torch.empty_like(base), torch.empty_like(base)
     k_max = torch.empty(1, dtype=torch.int32, device=base.device)
     stream = torch.cuda.current_stream(base.device).cuda_stream

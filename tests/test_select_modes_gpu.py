@@ -141,3 +141,22 @@ def test_selection_budgets_match_oracle(cuda_device, L, n_sink, rows, hi):
         want = selection_counts_ref(L, n_sink, 128, eff).clamp(max=L).to(torch.int32)
         b, t, m = selection_budgets(L, n_sink, 128, base.to(cuda_device), None if fr is None else fr.to(cuda_device), fa)
         assert torch.equal(b.cpu(), want) and torch.equal(t.cpu(), want // 128) and m == int(want.max())
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32, torch.int16])
+def test_selection_budgets_take_what_selection_counts_takes(cuda_device, dtype):
+    """Any integer type, strided tensors, counts beyond the row; what the kernel cannot read is refused."""
+    from mcsparse_b200.kernels.flash_mcsa.token_sparse import selection_budgets, selection_counts
+    L, n_sink = 5000, 4
+    base = torch.randint(0, 6000, (2, 3, 14), generator=torch.Generator().manual_seed(2)).to(dtype)
+    base[0, 0, 0] = torch.iinfo(dtype).max
+    base[1, 2, 4] = -7
+    want = selection_counts(L, n_sink, 128, base[..., ::2]).to(torch.int32)
+    b, t, m = selection_budgets(L, n_sink, 128, base.to(cuda_device)[..., ::2])
+    assert b.dtype == t.dtype == torch.int32 and b.shape == want.shape
+    assert torch.equal(b.cpu(), want) and torch.equal(t.cpu(), want // 128) and m == int(want.max())
+    rows = torch.full((2, 3, 7), 700, dtype=dtype)
+    want = selection_counts(L, n_sink, 128, torch.maximum(base[..., ::2], rows)).to(torch.int32)
+    assert torch.equal(selection_budgets(L, n_sink, 128, base.to(cuda_device)[..., ::2], rows.to(cuda_device))[0].cpu(), want)
+    with pytest.raises(ValueError):
+        selection_budgets(L, n_sink, 128, base.to(cuda_device), rows.to(cuda_device))

@@ -272,26 +272,33 @@ int mcs_topk_select_var(const float* scores, int32_t* out, const int32_t* sinks,
 /*
  * Top-p budgets: counts[r] = number of leading tokens of row r, in descending order of score, whose scores summed
  * BEFORE each of them stay below topp (at least 1, everything if the row's total stays below topp); sink tokens are
- * left out of the ranking and of the count.  scores: (rows, L) fp32 normalised masses; 0 < topp <= 1.
+ * left out of the ranking and of the count.  scores: (rows, L) fp32 normalised masses; 0 < topp <= 1; sinks distinct.
  *
  * Replaces: the sort + cumulative sum + mask count of mcsparse/kernels/flash_mcsa/token_sparse.py:842-852 and
- * :862-866 (topp / topk_topp modes); the tile alignment and the lower bound of topk_topp stay on the host.
+ * :862-866 (topp / topk_topp modes); mcs_selection_budgets turns the counts into budgets.
  */
-/* The same two with the sink positions in host memory (read during the call; each in [0, L)): no copy to the device.
- * k_rows may be NULL. */
+int mcs_topp_count(const float* scores, const int32_t* sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
+                   int32_t* counts, void* stream);
+
+/*
+ * The selection and the top-p count with the sink positions in host memory: read during the call, so there is no copy of the
+ * list to the device and the call may be captured.  Positions outside [0, L) and repeated ones are MCS_ERR_BAD_SHAPE.
+ * k_rows may be NULL (one budget for all rows).
+ */
 int mcs_topk_select_host_sinks(const float* scores, int32_t* out, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L,
                                int32_t k_total, const int32_t* k_rows, void* stream);
 int mcs_topp_count_host_sinks(const float* scores, const int32_t* host_sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
                               int32_t* counts, void* stream);
+
 /*
- * Budgets of the variable-length modes (token_sparse.py:811-823, :902-923) from ranked counts, all in device memory: per row
- * max(base, floor_rows or floor_all, 1) in whole tiles (at most L), plus the sinks, in whole tiles again; budgets in
- * tokens, tiles = budgets / tile, k_max = the largest budget.
+ * Budgets of the variable-length modes from ranked counts, all in device memory: per row max(base, floor_rows or floor_all, 1)
+ * in whole tiles (at most L), plus the sinks, in whole tiles again as long as tokens are left to fill them; budgets in tokens,
+ * tiles = budgets / tile, k_max = the largest budget.  floor_rows may be NULL.
+ *
+ * Replaces: the tile alignment and the lower bound of topk_topp, mcsparse/kernels/flash_mcsa/token_sparse.py:811-823, :902-923.
  */
 int mcs_selection_budgets(const int32_t* base, const int32_t* floor_rows, int32_t floor_all, int64_t rows, int32_t L, int32_t n_sink,
                           int32_t tile, int32_t* budgets, int32_t* tiles, int32_t* k_max, void* stream);
-int mcs_topp_count(const float* scores, const int32_t* sinks, int32_t n_sink, int64_t rows, int32_t L, float topp,
-                   int32_t* counts, void* stream);
 
 /*
  * Fast PDDP query grouping: per (batch*head) permutation that puts similar rows into aligned

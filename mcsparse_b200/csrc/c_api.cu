@@ -25,11 +25,14 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 static long long* g_clock_out = nullptr;
 
-// copies a host list of sink positions into the launch's argument block; false if one lies outside the row
+// copies a host list of sink positions into the launch's argument block; false if one lies outside the row or comes twice
+// (the selection counts on n different sinks, the top-p count takes each sink's score out once)
 static bool sink_list(const int32_t* host_sinks, int n, int L, mcs::SinkList& out) {
   if (host_sinks == nullptr) return true;
   for (int i = 0; i < n; ++i) {
     if (host_sinks[i] < 0 || host_sinks[i] >= L) return false;
+    for (int j = 0; j < i; ++j)
+      if (host_sinks[j] == host_sinks[i]) return false;
     out.idx[i] = host_sinks[i];
   }
   return true;

@@ -155,9 +155,11 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const __grid_c
     }
     if (lane == 0) { sh.warp_sel[warp] = c_sel; sh.warp_eq[warp] = c_eq; }
     __syncthreads();
-    int eq_before = 0, out_before = 0;
-    for (int w = 0; w < warp; ++w) {                       // 32 entries: a serial prefix is cheapest
+    int eq_before = 0, out_before = 0, n_out = need;       // (repeated sinks, which the contract excludes: fewer than k_row)
+    for (int w = 0; w < kWarps; ++w) {                     // 32 entries: a serial prefix is cheapest
       const int e = sh.warp_eq[w];
+      n_out += sh.warp_sel[w];
+      if (w >= warp) continue;
       out_before += sh.warp_sel[w] + min(max(need - eq_before, 0), e);
       eq_before += e;
     }
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const __grid_c
       eq_before += __popc(eq_b);
       out_before += __popc(sel_b);
     }
-    for (int i = k_row + tid; i < p.k_total; i += kThreads) out[i] = 0;      // beyond the row's own budget: padding
+    for (int i = min(k_row, n_out) + tid; i < p.k_total; i += kThreads) out[i] = 0;      // beyond the row's own budget: padding
     __syncthreads();                                       // shared state is reused by the next row
   }
 }
@@ -510,18 +512,20 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_co
         prefix16[w] = (uint16_t)before;
         before += __popc(bm[w]);
       }
+      if (tid == kST - 1) sh.rem = before;                         // indices in all
       __syncthreads();
+      const int n_out = min(k_row, (int)sh.rem);                   // (repeated sinks, which the contract excludes: fewer than k_row)
       for (int w = tid; w < words; w += kST) {
         uint32_t b = bm[w];
         int pos = prefix16[w];
         while (b != 0u) {
-          if (pos < k_row) ckeys[pos] = (uint32_t)(w * 32 + __ffs((int)b) - 1);
+          if (pos < n_out) ckeys[pos] = (uint32_t)(w * 32 + __ffs((int)b) - 1);
           ++pos;
           b &= b - 1u;
         }
       }
       __syncthreads();
-      for (int i = tid; i < p.k_total; i += kST) out[i] = i < k_row ? (int)ckeys[i] : 0;   // beyond the row's budget: padding
+      for (int i = tid; i < p.k_total; i += kST) out[i] = i < n_out ? (int)ckeys[i] : 0;   // beyond the row's budget: padding
     }
   }
 }

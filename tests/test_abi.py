@@ -40,6 +40,18 @@ def test_argument_errors_without_a_gpu():
     assert lib.mcs_perm_apply(None, None, None, 1, 1, 16, 16, 16, 16, 16, None) == -1
 
 
+def test_host_sink_lists_are_checked():
+    """Sink positions in host memory: inside the row and different from one another (the kernels count on it)."""
+    import ctypes as C
+    from mcsparse_b200 import _lib
+    lib = _lib.lib()
+    scores = out = C.c_void_p(0x1000)                                     # never touched: every call below is refused on the host
+    for bad in ((0, 1, 1, 3), (5, 5), (9, 0, 2, 9), (0, 10), (-1, 2)):
+        sinks = (C.c_int32 * len(bad))(*bad)
+        assert lib.mcs_topk_select_host_sinks(scores, out, sinks, len(bad), 1, 10, 6, None, None) == -2, bad
+        assert lib.mcs_topp_count_host_sinks(scores, sinks, len(bad), 1, 10, 0.5, out, None) == -2, bad
+
+
 def test_wrappers_fail_loudly_without_cuda():
     import pytest
     import torch

@@ -136,3 +136,18 @@ def test_threads_with_different_row_lengths(cuda_device):
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not errors, errors
+
+
+@pytest.mark.parametrize("L,k_total", [(300, 128), (9000, 1024), (32760, 28000)])          # streaming kernel (two forms), general kernel
+def test_repeated_sinks_leave_no_foreign_entries(cuda_device, L, k_total):
+    """The device-list entry point cannot check its sinks on the host.  Repeated ones are outside its contract; the row then holds
+    fewer indices, ascending, and zeros behind them - nothing that was not written."""
+    from mcsparse_b200 import _lib
+    scores = torch.rand(5, L, generator=torch.Generator().manual_seed(L)) ** 8
+    sinks = torch.tensor([3, 7, 7, 7], dtype=torch.int32, device=cuda_device)
+    out = torch.full((5, k_total), 0x3F800000, dtype=torch.int32, device=cuda_device)
+    d = scores.to(cuda_device)
+    assert _lib.lib().mcs_topk_select(d.data_ptr(), out.data_ptr(), sinks.data_ptr(), 4, 5, L, k_total, torch.cuda.current_stream().cuda_stream) == 0
+    out = out.cpu()
+    want = select_topk_ref(scores, k_total - 2, sinks=[3, 7])
+    assert torch.equal(out[:, :k_total - 2], want) and bool((out[:, k_total - 2:] == 0).all())

@@ -149,7 +149,7 @@ def test_selection_budgets_take_what_selection_counts_takes(cuda_device, dtype):
     from mcsparse_b200.kernels.flash_mcsa.token_sparse import selection_budgets, selection_counts
     L, n_sink = 5000, 4
     base = torch.randint(0, 6000, (2, 3, 14), generator=torch.Generator().manual_seed(2)).to(dtype)
-    base[0, 0, 0] = torch.iinfo(dtype).max
+    base[0, 0, 0] = min(torch.iinfo(dtype).max, 2**40)
     base[1, 2, 4] = -7
     want = selection_counts(L, n_sink, 128, base[..., ::2]).to(torch.int32)
     b, t, m = selection_budgets(L, n_sink, 128, base.to(cuda_device)[..., ::2])

@@ -255,8 +255,9 @@ __device__ __forceinline__ void hist_find(SharedStream& sh, uint32_t kr) {
 // Key of the k-th largest key among those that visit(f) hands to f (key 0: not counted; the others lie in [lo, hi]);
 // `need` of the `n_eq` keys equal to it belong to the k largest.  Passes of 11 bits over the bits in which the keys
 // differ at all, so that the first histogram already spreads over its bins; at most max_passes (the result is then
-// a lower bound: its remaining bits are zero).  Needs a cleared histogram.
-template <typename Visit>
+// a lower bound: its remaining bits are zero).  Needs a cleared histogram.  kWhole: f is called by whole warps, and keys of
+// one digit are counted together (for whole rows, which may be one single tie group).
+template <bool kWhole = false, typename Visit>
 __device__ __forceinline__ void kth_key(SharedStream& sh, uint32_t k, uint32_t lo, uint32_t hi, int max_passes, Visit visit, uint32_t& T,
                                         uint32_t& need, uint32_t& n_eq) {
   const int bits = 32 - __clz((int)(hi - lo));
@@ -267,8 +268,17 @@ __device__ __forceinline__ void kth_key(SharedStream& sh, uint32_t k, uint32_t l
   for (int pass = 0; pass < max_passes; ++pass) {
     visit([&](uint32_t key) {
       const uint32_t x = key - lo;
-      if (key != 0u && (above == 32 || (x >> above) == prefix))
-        atomicAdd(&sh.hist[(above == 32 ? x >> shift : (x >> shift) & ((1u << (above - shift)) - 1u))], 1u);
+      const bool live = key != 0u && (above == 32 || (x >> above) == prefix);
+      const uint32_t digit = above == 32 ? x >> shift : (x >> shift) & ((1u << (above - shift)) - 1u);
+      if constexpr (kWhole) {
+        const uint32_t lanes = __ballot_sync(0xffffffffu, live);
+        if (live) {
+          const uint32_t peers = __match_any_sync(lanes, digit);
+          if (__ffs((int)peers) - 1 == (int)(threadIdx.x & 31)) atomicAdd(&sh.hist[digit], (uint32_t)__popc(peers));
+        }
+      } else if (live) {
+        atomicAdd(&sh.hist[digit], 1u);
+      }
     });
     __syncthreads();
     hist_find(sh, k);
@@ -433,7 +443,17 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_co
         live = C - sh.n_dead;
       }
       auto row_key = [&](int j) { return is_sink(j) ? 0u : score_key(__ldg(sc + j)); };
-      auto visit_row = [&](auto f) { for (int j = tid; j < L; j += kST) f(row_key(j)); };
+      // (whole warps, four keys of a thread in flight)
+      auto visit_row = [&](auto f) {
+#pragma unroll 1
+        for (int j0 = tid & ~31; j0 < L; j0 += 4 * kST) {
+          uint32_t key[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) { const int j = j0 + u * kST + lane; key[u] = j < L ? row_key(j) : 0u; }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) f(key[u]);
+        }
+      };
       if (live >= (uint32_t)k) {
         kth_key(sh, (uint32_t)k, sh.key_lo, sh.key_hi, 3, [&](auto f) { for (int i = tid; i < (int)C; i += kST) f(ckeys[i]); }, T, need, n_eq);
       } else {
@@ -451,15 +471,18 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_co
           T = t_key;
           need = (uint32_t)k - live;
         }
-        if (!tie) kth_key(sh, (uint32_t)k, 0u, 0xFFFFFFFFu, 3, visit_row, T, need, n_eq);
+        if (!tie) kth_key<true>(sh, (uint32_t)k, 0u, 0xFFFFFFFFu, 3, visit_row, T, need, n_eq);
       }
       // ---- 4. bitmap of the selected keys: above T, and the `need` lowest indices among those equal to T
       auto mark = [&](bool above, bool equal) {
         if (from_row) {
           // (keys of the row are compared without the sink test, whose bits may be gone: a sink belongs to the result)
-          for (int j = tid; j < L; j += kST) {
-            const uint32_t key = score_key(__ldg(sc + j));
-            if ((above && key > T) || (equal && key == T)) set_bit(j);
+          // one word of the bitmap per warp and step
+#pragma unroll 4
+          for (int j0 = tid & ~31; j0 < L; j0 += kST) {
+            const uint32_t key = j0 + lane < L ? score_key(__ldg(sc + j0 + lane)) : 0u;      // (no score has key 0, and T is not 0)
+            const uint32_t word = __ballot_sync(0xffffffffu, (above && key > T) || (equal && key == T));
+            if (lane == 0 && word != 0u) atomicOr(&bm[j0 >> 5], word);
           }
         } else {
           for (int i = tid; i < (int)C; i += kST) {

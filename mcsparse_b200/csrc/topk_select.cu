@@ -255,9 +255,9 @@ __device__ __forceinline__ void hist_find(SharedStream& sh, uint32_t kr) {
 // Key of the k-th largest key among those that visit(f) hands to f (key 0: not counted; the others lie in [lo, hi]);
 // `need` of the `n_eq` keys equal to it belong to the k largest.  Passes of 11 bits over the bits in which the keys
 // differ at all, so that the first histogram already spreads over its bins; at most max_passes (the result is then
-// a lower bound: its remaining bits are zero).  Needs a cleared histogram.  kWhole: f is called by whole warps, and keys of
-// one digit are counted together (for whole rows, which may be one single tie group).
-template <bool kWhole = false, typename Visit>
+// a lower bound: its remaining bits are zero).  Needs a cleared histogram.  (Equal keys cost no more than others: the
+// hardware counts the lanes of an increment that hit one bin together.)
+template <typename Visit>
 __device__ __forceinline__ void kth_key(SharedStream& sh, uint32_t k, uint32_t lo, uint32_t hi, int max_passes, Visit visit, uint32_t& T,
                                         uint32_t& need, uint32_t& n_eq) {
   const int bits = 32 - __clz((int)(hi - lo));
@@ -270,15 +270,7 @@ __device__ __forceinline__ void kth_key(SharedStream& sh, uint32_t k, uint32_t l
       const uint32_t x = key - lo;
       const bool live = key != 0u && (above == 32 || (x >> above) == prefix);
       const uint32_t digit = above == 32 ? x >> shift : (x >> shift) & ((1u << (above - shift)) - 1u);
-      if constexpr (kWhole) {
-        const uint32_t lanes = __ballot_sync(0xffffffffu, live);
-        if (live) {
-          const uint32_t peers = __match_any_sync(lanes, digit);
-          if (__ffs((int)peers) - 1 == (int)(threadIdx.x & 31)) atomicAdd(&sh.hist[digit], (uint32_t)__popc(peers));
-        }
-      } else if (live) {
-        atomicAdd(&sh.hist[digit], 1u);
-      }
+      if (live) atomicAdd(&sh.hist[digit], 1u);
     });
     __syncthreads();
     hist_find(sh, k);
@@ -421,7 +413,7 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_co
       // ---- 3. the exact k-th key
       const uint32_t C = sh.n_cand;
       uint32_t T = 0u, need = 0u, n_eq = 0u;
-      bool from_row = false;
+      bool from_row = false, tie = false;
       uint32_t live = 0;
       if (C <= (uint32_t)cap) {
         uint32_t lo = 0xFFFFFFFFu, hi = 0u;
@@ -442,27 +434,27 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_co
         __syncthreads();
         live = C - sh.n_dead;
       }
-      auto row_key = [&](int j) { return is_sink(j) ? 0u : score_key(__ldg(sc + j)); };
-      // (whole warps, four keys of a thread in flight)
+      // f(index, key) for the whole row, by whole warps (key 0 beyond its end), four loads of a thread in flight: what bounds these
+      // passes is the latency of L2
       auto visit_row = [&](auto f) {
 #pragma unroll 1
         for (int j0 = tid & ~31; j0 < L; j0 += 4 * kST) {
-          uint32_t key[4];
+          float v[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) { const int j = j0 + u * kST + lane; key[u] = j < L ? row_key(j) : 0u; }
+          for (int u = 0; u < 4; ++u) { const int j = j0 + u * kST + lane; v[u] = j < L ? __ldg(sc + j) : 0.f; }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) f(key[u]);
+          for (int u = 0; u < 4; ++u) { const int j = j0 + u * kST + lane; f(j, j < L ? score_key(v[u]) : 0u); }
         }
       };
+      auto ranked = [&](int j, uint32_t key) { return key == 0u || is_sink(j) ? 0u : key; };
       if (live >= (uint32_t)k) {
         kth_key(sh, (uint32_t)k, sh.key_lo, sh.key_hi, 3, [&](auto f) { for (int i = tid; i < (int)C; i += kST) f(ckeys[i]); }, T, need, n_eq);
       } else {
         from_row = true;
-        bool tie = false;
         if (sampled && C <= (uint32_t)cap) {
           // a tie group on the bound itself (masses that underflow to zero): the k-th key is t
           uint32_t n = 0;
-          visit_row([&](uint32_t key) { n += (key == t_key) ? 1u : 0u; });
+          visit_row([&](int j, uint32_t key) { n += (key == t_key && !is_sink(j)) ? 1u : 0u; });
           n = __reduce_add_sync(0xffffffffu, n);
           if (lane == 0) atomicAdd(&sh.n_tie, n);
           __syncthreads();
@@ -471,20 +463,19 @@ __global__ void __launch_bounds__(kST, kCtas) topk_stream_kernel(const __grid_co
           T = t_key;
           need = (uint32_t)k - live;
         }
-        if (!tie) kth_key<true>(sh, (uint32_t)k, 0u, 0xFFFFFFFFu, 3, visit_row, T, need, n_eq);
+        if (!tie)
+          kth_key(sh, (uint32_t)k, 0u, 0xFFFFFFFFu, 3, [&](auto f) { visit_row([&](int j, uint32_t key) { f(ranked(j, key)); }); }, T, need, n_eq);
       }
       // ---- 4. bitmap of the selected keys: above T, and the `need` lowest indices among those equal to T
       auto mark = [&](bool above, bool equal) {
-        if (from_row) {
-          // (keys of the row are compared without the sink test, whose bits may be gone: a sink belongs to the result)
-          // one word of the bitmap per warp and step
-#pragma unroll 4
-          for (int j0 = tid & ~31; j0 < L; j0 += kST) {
-            const uint32_t key = j0 + lane < L ? score_key(__ldg(sc + j0 + lane)) : 0u;      // (no score has key 0, and T is not 0)
+        // (keys of the row are compared without the sink test, whose bits may be gone: a sink belongs to the result; a tie
+        // group on the bound: the keys above it are the candidates)
+        if (from_row && (equal || !tie))
+          visit_row([&](int j, uint32_t key) {                   // one word of the bitmap per warp and step
             const uint32_t word = __ballot_sync(0xffffffffu, (above && key > T) || (equal && key == T));
-            if (lane == 0 && word != 0u) atomicOr(&bm[j0 >> 5], word);
-          }
-        } else {
+            if (lane == 0 && word != 0u) atomicOr(&bm[j >> 5], word);
+          });
+        if (!from_row || (tie && above)) {
           for (int i = tid; i < (int)C; i += kST) {
             const uint32_t key = ckeys[i];
             if ((above && key > T) || (equal && key == T)) set_bit(cidx[i]);

@@ -125,11 +125,25 @@ def test_mass_other_head_dims(cuda_device, D):
     assert torch.equal(out1, group_mass(q.to(dev), kd.contiguous(), lse1.to(dev)).cpu().double())
 
 
-# two groups per CTA (D = 128): odd numbers of groups, short groups, key stretches of unequal length
-@pytest.mark.parametrize("B,H,Lq,Lk,rows", [(1, 12, 3400, 2000, 128), (1, 40, 1200, 1100, 128), (2, 9, 2000, 900, 64), (1, 1, 130, 5000, 128),
-                                            (1, 148, 300, 130, 128)])
-def test_two_groups_per_cta(cuda_device, B, H, Lq, Lk, rows):
+def _ctas_per_pair(bh, M, Lk):
+    """The kernel's choice at D = 128: CTAs per pair of groups, 0 for one group per CTA (the cost in group_mass.cu)."""
+    sms, tiles = torch.cuda.get_device_properties(0).multi_processor_count, -(-Lk // 128)
+    best, splits = -(-bh * M // sms) * (tiles + 4.0), 0
+    for s in range(1, min(8, tiles) + 1):
+        cost = -(-bh * ((M + 1) // 2) * s // sms) * (-(-tiles // s) * 1.9 + 4.0)
+        if cost < best:
+            best, splits = cost, s
+    return splits
+
+
+# two groups per CTA (D = 128): odd numbers of groups, short groups, key stretches of unequal length.  The first group is done again
+# by itself; where the two launches take different forms (``both``), the forms are seen to add in the same order.
+@pytest.mark.parametrize("B,H,Lq,Lk,rows,both", [(1, 12, 3400, 2000, 128, False), (1, 40, 1200, 1100, 128, True), (2, 9, 2000, 900, 64, False),
+                                                 (1, 1, 130, 5000, 128, False), (1, 148, 300, 130, 128, True), (1, 100, 256, 1500, 128, True),
+                                                 (2, 40, 250, 700, 64, True)])
+def test_two_groups_per_cta(cuda_device, B, H, Lq, Lk, rows, both):
     from mcsparse_b200.kernels.flash_mcsa.token_sparse import group_mass
+    assert ((_ctas_per_pair(B * H, -(-Lq // rows), Lk) > 0) != (_ctas_per_pair(B * H, 1, Lk) > 0)) == both
     g = torch.Generator().manual_seed(Lq + Lk)
     q = torch.randn(B, H, Lq, 128, generator=g).to(torch.bfloat16).to(cuda_device)
     k = torch.randn(B, H, Lk, 128, generator=g).to(torch.bfloat16).to(cuda_device)
@@ -143,6 +157,6 @@ def test_two_groups_per_cta(cuda_device, B, H, Lq, Lk, rows):
         want = p[:, :, m * rows:(m + 1) * rows].mean(2)
         err = (got[:, :, m] - want).abs() / want.abs().clamp_min(1e-7)
         assert float(err.max()) < 2e-3, (m, float(err.max()))          # the tolerance of the tests above
-    # the first group alone (one group per CTA): the same bits
+    # the first group alone: the same bits
     q0 = q.gather(2, idx[:, :, :rows].expand(B, H, min(rows, Lq), 128))
     assert torch.equal(group_mass(q0, k, lse[:, :, :rows], group_rows=rows, normalize=True)[:, :, 0], got[:, :, 0])

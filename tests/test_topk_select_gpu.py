@@ -53,17 +53,22 @@ def test_reference_shaped_wrapper(cuda_device):
     assert torch.equal(gi2.cpu(), select_topk_ref(tp, 256))
 
 
-@pytest.mark.parametrize("L", [32768, 32761, 4100])
-def test_register_path_structured_rows(cuda_device, L):
-    """Rows that defeat the sampled lower bound of the register-resident kernel (it must only cost time):
-    ramps, the winners hidden between the sampled positions, NaN-heavy and constant rows, a few NaNs."""
+@pytest.mark.parametrize("L", [32768, 32761, 8193, 4100])
+def test_rows_that_mislead_the_sample(cuda_device, L):
+    """Rows that defeat the sampled lower bound of the streaming kernel (it must only cost time): one key in L / 4096 is sampled in
+    rows of more than 8,192.  Winners at the sampled positions alone (the bound is too high: fewer candidates than wanted) and
+    everywhere but there (too low: more than fit); ramps, NaN-heavy and constant rows, a few NaNs."""
     g = torch.Generator().manual_seed(L)
     k_total = 2048 if L > 5000 else 512
     rows = []
     rows.append(torch.arange(L).float())                                   # winners at the end
     rows.append(torch.arange(L, 0, -1).float())                            # winners at the start
-    hidden = torch.zeros(L)
-    pos = torch.arange(1, L, 4)[: k_total + 100]                           # never a sampled position (those are multiples of 4)
+    sampled = torch.zeros(L, dtype=torch.bool)
+    sampled[torch.arange(4096) * L // 4096] = True
+    rows.append(torch.rand(L, generator=g) * 0.5 + sampled)                # too few above the bound
+    rows.append(torch.rand(L, generator=g) * 0.5 + ~sampled)               # (L > 8,192) everything not sampled above the bound
+    hidden = torch.zeros(L)                                                # no winner sampled: the bound is the zeros' tie group
+    pos = (~sampled if L > 8192 else sampled | ~sampled).nonzero().flatten()[: k_total + 100]
     hidden[pos] = 1.0 + torch.rand(pos.numel(), generator=g)
     rows.append(hidden)
     nan_row = torch.rand(L, generator=g)

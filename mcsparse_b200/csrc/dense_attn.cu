@@ -24,11 +24,11 @@
 // What bounds it: per pair of tiles the tensor pipe needs 2,048 cycles and the special-function unit the same
 // (32,768 exponentials at 16 per clock); under a long load the GPU's power limit lowers the clock.  Measured at 24 heads x
 // 32,760 x 128 bf16 (13.2 TFLOP; 8.0 ms at the measured burst rate, 9.4 at the sustained one): 11.24 -> 10.14 ms in short
-// bursts, 12.98 -> 11.54 ms in a long loop (3,146 cycles per pair of tiles; 1.77 GHz in a burst, 1.51 GHz in the loop).
+// bursts, 12.85 -> 11.28 ms in a loop of calls (3,146 cycles per pair of tiles; 1.77 GHz in a burst, 1.51 GHz in the loop).
 // The exponentials are not what is left: without any (results wrong, timing only) a pair takes 3,225 cycles against 3,260
 // before P V started early.  Shared memory is as busy as the tensor pipe: Q K^T reads both operands from it at 128 bytes
 // per cycle, its full rate, while the next tiles are written.  Measured and not kept: an eighth / a quarter of the
-// exponentials as polynomials on the FMA pipe (12.18 / 12.19 ms against 11.67 in the loop: issue slots and energy), scalar
+// exponentials as polynomials on the FMA pipe (12.18 / 12.19 ms against 11.67 measured beside them in a loop: issue slots and energy), scalar
 // instead of two-wide fused multiply-adds (12.13), P V started at half of the tile (11.60 against 11.54 at three quarters).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

@@ -23,11 +23,12 @@
 // out of the same buffer.  The softmax of tile g+1 thus finds its scores ready and never waits for a product.
 // What bounds it: the softmax of a tile (two warps per sub-partition) and the row gather, 256 rows of 2 D bytes per tile.
 // With four softmax warps over whole rows and one score buffer a tile took 4,900 cycles at every head dimension.
-// Measured (8 heads x 20,475 tokens, 3,072 selected, permutation and residual): D = 144 fp16 580 -> 471 us (290 GFLOP;
-// 176 us at the measured burst rate), 96 418 -> 371, 160 574 -> 522, 192 581 -> 556, 256 687 -> 664, e4m3 160 395 -> 354
-// (the rule by whole rows costs 2 us of it).
-// Every mbarrier wait is bounded and reports through the status
-// word; a role whose wait expires leaves its loop, the others follow through their own bounded waits.
+// Measured (8 heads x 20,475 tokens, 3,072 selected, permutation and residual; device time of a replayed graph): D = 144
+// 535 -> 420 us (290 GFLOP; 176 us at the measured burst rate), 32 287 -> 253, 96 375 -> 325, 160 533 -> 482, 192 541 -> 515,
+// 256 660 -> 641; e4m3 16 265 -> 263, 96 334 -> 305, 160 394 -> 354, 256 426 -> 388 (two less at 160 with the reference point
+// by half rows, which gives other outputs).
+// Every mbarrier wait is bounded and reports through the status word; a role whose wait expires leaves its loop, the others
+// follow through their own bounded waits.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -533,7 +534,8 @@ int launch_wide(const GatherAttnParams& p, cudaStream_t stream) {
 int launch_gather_attn_wide(const GatherAttnParams& p, bool fp16, cudaStream_t stream) {
   if (p.D < 8 || p.D > 256 || p.D % 8 != 0 || p.group_rows > 128) return -3;
   // 144 and 160: a quarter and a sixth of the copies of the block-wise gather would be padding (144: 471 us against 548;
-  // 160: 522 against 548).  At 96 the block-wise gather wins (371 against 389), as for the 160-byte rows of e4m3 (389 / 402).
+  // 160: 522 against 548, in a loop of calls).  At 96 the block-wise gather wins (371 against 389), as for the 160-byte rows of
+  // e4m3 (389 / 402).
   if (p.D == 144) return fp16 ? launch_wide<3, 1, 18>(p, stream) : launch_wide<3, 0, 18>(p, stream);
   if (p.D == 160) return fp16 ? launch_wide<3, 1, 20>(p, stream) : launch_wide<3, 0, 20>(p, stream);
   const int nb = (p.D + 63) / 64;

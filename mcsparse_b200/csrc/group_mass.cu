@@ -19,8 +19,9 @@
 // columns are (1, 1, 1, 0, ...) and whose Q columns are (-hi, -mid, -lo, 0, ...), a three-term
 // bf16 split of lse_i / scale, exact to fp32 precision.  The tensor core then delivers
 // q_i . k_j - lse_i / scale and each element costs one multiply, one ex2 and one add.
-// The kernel is bound by the ex2 throughput of the SFU (16 per clock per SM); a quarter of the exponentials
-// are therefore evaluated by a polynomial on the FMA pipe.
+// The SFU delivers 16 ex2 per clock and SM; a quarter of the exponentials are therefore evaluated by a polynomial on the FMA
+// pipe.  With two query groups per CTA the SFU is busy 74% of the time, the tensor pipe 56%, and the products read both
+// operands from shared memory at its full rate.
 //
 // Roles: warps 0-15 exponentiate and sum, in two groups of eight for the even and the odd key tiles, or for the two query
 // groups (two threads per key token: warps w and w+4 of a group share a TMEM lane group and take 64 query columns each; the two partial sums meet in
@@ -246,10 +247,10 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
       }
       tc_fence_before();
       const float sum = (a0 + a1) + (a2 + a3);
-      // The two halves of a row meet in shared memory, double-buffered by tile parity and handed over
+      // The two halves of a row meet in shared memory, in one place per score buffer, and are handed over
       // through an mbarrier (a bounded wait, unlike a named barrier).  The lower half releases the score
-      // buffer only after it has read the partner's sums, so the partner's write two tiles later (which
-      // needs that release to get its next scores) cannot overtake the read.  (Copying all 64 values to
+      // buffer only after it has read the partner's sums, so the partner's next write to that place (which
+      // needs the release to get the buffer's next scores) cannot overtake the read.  (Copying all 64 values to
       // registers first and releasing the score buffer before the exponentials measured 10% slower.)
       if (x == 1) {
         part[pb * 128 + j_in] = sum;
@@ -384,6 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
   }
 }
 
+// (splits: for pairs of groups, see pair_splits; a single group takes all of its head's keys)
 template <int D, bool kFp16, int G = 1>
 int launch(const GroupMassParams& p, cudaStream_t stream, int splits = 1) {
   using L = Smem<D, G>;

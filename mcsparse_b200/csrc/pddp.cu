@@ -273,7 +273,7 @@ __device__ __forceinline__ void project_rows(uint32_t s_base, int warp, int lane
 // writes column d and every store is one 128-byte line per warp.
 // Same sums in the same order as a kernel per stage had: identical permutations.
 // Measured (24 heads x 32,760 tokens x 128, 8 levels, kernel times of one call): Gram 1,140 + power 638 + project 556 us
-// before; node 599 + power 62 + project 196 us now (X read twice per level at the measured copy rate: 490 us).  Of that,
+// before; node 581 + power 63 + project 192 us now (X read twice per level at the measured copy rate: 490 us).  Of that,
 // lanes that load whole rows instead of a row each, the transposed partial store and the fused power step are the most.
 // ------------------------------------------------------------------------------------------
 template <int D, bool kFp16>

@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(kThreads, 1) topk_select_kernel(const __grid_c
 // which warps append candidates does not matter.  A row on which the sample misjudges (fewer than k keys above t and
 // not the tie group at t itself, or more candidates than fit) is selected by the same passes over global memory: the
 // sample decides the time only, never the result.
-// Measured (one B200): 3,840 rows of 98,280 keys, k = 4,096: 8,089 -> 673 us (1.57 GB, floor 240 us at the measured copy
-// rate).  The sweep itself runs at 5.5 TB/s; the other half of a row's time are the sample and histogram passes.
+// Measured (one B200, a loop of calls with four sinks): 3,840 rows of 98,280 keys, k = 4,096: 8,058 -> 640 us (1.57 GB, floor
+// 240 us at the measured copy rate).  The sweep itself runs at 5.5 TB/s; the other half of a row's time are the sample and histogram passes.
 // ------------------------------------------------------------------------------------------
 constexpr int kST = 512;                  // threads of the streaming kernel
 constexpr int kSW = kST / 32;
@@ -554,14 +554,17 @@ int launch_topk_select(const TopkParams& p, cudaStream_t stream) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // Streaming path whenever the candidates that the sampled bound lets through fit in shared memory beside the bitmap, even
-  // if only one CTA fits.  Measured against the kernels it replaced (general above 32,768 keys, a register-resident one below):
-  //   rows x keys, k          before   streaming
-  //   3,840 x 98,280, 4,096   8,089     673 us        6,144 x 32,760, 2,048     921     480 us
-  //   2,000 x 98,280, 8,192   4,378     596           6,144 x 32,760, 8,192   5,928     780
-  //   1,500 x 60,000, 13,000  2,137     462           3,000 x 32,760, 20,000  3,043     895
-  //   444 x 4,700, 1,280        104      58           1,024 x 16,380, 1,664     179      92
-  // (three CTAs per SM with two loads each against two with four: 480 / 491 us at 32,760 keys, 58 / 65 at 4,700; where only
-  // two fit, four loads win: 673 / 723 at 98,280).  Beyond it the general kernel: 2,000 x 32,760, k = 28,000 in 720 us.
+  // if only one CTA fits.  Against the kernels it replaced (general above 32,768 keys, a register-resident one below), masses
+  // with a tenth of zeros, no sinks, device time of a replayed graph in us:
+  //   rows x keys, k          before   streaming        rows x keys, k          before   streaming
+  //   3,840 x 98,280, 4,096    6,353     637            6,144 x 32,760, 2,048     882     457
+  //   2,000 x 98,280, 8,192    3,447     561            6,144 x 32,760, 8,192   4,575     759
+  //   1,500 x 60,000, 13,000   1,680     431            3,000 x 32,760, 20,000  2,350     861
+  //   444 x 4,700, 1,280          67      23            1,024 x 16,380, 1,664     143      59
+  // (three CTAs per SM with two loads each against two with four, in an earlier loop of calls: 480 / 491 at 32,760 keys, 58 / 65
+  // at 4,700; where only two fit, four loads win: 673 / 723 at 98,280).  Beyond it the general kernel: 2,000 x 32,760,
+  // k = 28,000 in 638.  What the sample cannot help with is dearer than on the staged row of the general kernel where one CTA
+  // fits: 600 x 40,000, k = 20,000 on rows of one single value 468 (273 there), of values 1e-5 apart 435 (373), on ramps 275 (244).
   if (p.L <= kStreamMaxL) {
     const int k = p.k_total - p.n_sink;
     const bool all = p.L <= kSampleAll;

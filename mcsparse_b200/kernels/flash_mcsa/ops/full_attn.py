@@ -43,7 +43,8 @@ def _dense(q: Tensor, k: Tensor, v: Tensor, scale: Optional[float], want_lse: bo
     B, H, Lq, D = q.shape
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    out = torch.empty_like(q)
+    # (in q's layout where its rows are contiguous: the kernel writes whole rows)
+    out = torch.empty_like(q) if q.stride(-1) == 1 else torch.empty(q.shape, dtype=q.dtype, device=q.device)
     lse = torch.empty(B, H, Lq, dtype=torch.float32, device=q.device) if want_lse else None
     qv, kv, vv, ov = (itf.maybe_contiguous(t).transpose(1, 2) for t in (q, k, v, out))   # (B, L, H, D) views
     residual, perm = itf._extras_checks(residual, perm, qv, q.dtype, B, H, Lq, D)

@@ -149,3 +149,12 @@ def test_dense_maximum_rises_from_tile_to_tile(cuda_device, dtype, D, levels, H)
     for _ in range(3):
         o2, l2 = full_attention_with_lse(qd, kd, vd)
         assert torch.equal(out, o2) and torch.equal(lse, l2)
+
+
+def test_dense_inputs_with_strided_rows(cuda_device):
+    """q, k, v whose last dimension is not the contiguous one: copied for the kernel, and the output is what the kernel wrote."""
+    from mcsparse_b200.kernels.flash_mcsa.ops.full_attn import full_attention
+    g = torch.Generator().manual_seed(9)
+    q, k, v = (torch.randn(1, 2, 64, n, generator=g).to(torch.bfloat16).to(cuda_device).transpose(2, 3) for n in (200, 300, 300))
+    assert q.stride(-1) != 1
+    assert torch.equal(full_attention(q, k, v), full_attention(q.contiguous(), k.contiguous(), v.contiguous()))

@@ -84,6 +84,68 @@ __device__ __forceinline__ uint32_t swz(int row, int c) {
   return static_cast<uint32_t>((c >> 3) * (kRows * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
 }
 
+// Constant extra K block, extra Q block and Q rows of tile rows row0 .. row0 + 31, by one warp.  (A function of its own: inlined
+// into the kernel, the same code costs the exponentiating loop 1%: 6,920 us against 6,840 at 24 heads x 32,760 x 128.)
+template <int D, bool kFp16, int G>
+__device__ __noinline__ void prepare_queries(uint8_t* smem, const float* lse, const int64_t* perm, const uint8_t* qb, size_t q_row, int m0,
+                                             int M, int group_rows, int Lq, float inv_scale, int d_chunks, int row0) {
+  using L = Smem<D, G>;
+  constexpr bool kWide = D > 128;
+  constexpr int kChunks = kWide ? 32 : D / 8;
+  constexpr int kRowsPerInstr = 32 / kChunks;
+  const int lane = threadIdx.x & 31, sub = lane / kChunks, cch = lane % kChunks;
+  const bool c_in_tile = !kWide || cch < D / 8;
+  const bool c_live = !kWide || cch < d_chunks;
+  const uint32_t s_base = smem_u32(smem);
+  // K extra: every row (1, 1, 1, 0, ...); Q extra: (-hi, -mid, -lo, 0, ...) of lse / scale
+  const uint32_t one = kFp16 ? 0x3C00u : 0x3F80u;
+  uint8_t* xt = smem + L::kX;
+  const int r = row0 + lane;
+  uint4 kv0 = make_uint4(one | (one << 16), one, 0, 0);
+  float x = 3.0e38f;                                 // padding rows: exp(-huge) = 0
+  if (kFp16) x = 60000.f;
+  const int m = m0 + (r >> 7), rr = r & 127, q_row0 = m * group_rows;
+  const int rows_valid = m < M ? min(group_rows, Lq - q_row0) : 0;
+  if (rr < rows_valid) x = lse[q_row0 + rr] * inv_scale;
+  uint32_t w0, w1;
+  if (kFp16) {
+    const __half hi = __float2half_rn(x);
+    const float r1 = x - __half2float(hi);
+    const __half mid = __float2half_rn(r1);
+    const __half lo = __float2half_rn(r1 - __half2float(mid));
+    w0 = (uint32_t)__half_as_ushort(__hneg(hi)) | ((uint32_t)__half_as_ushort(__hneg(mid)) << 16);
+    w1 = (uint32_t)__half_as_ushort(__hneg(lo));
+  } else {
+    const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+    const float r1 = x - __bfloat162float(hi);
+    const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
+    const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
+    w0 = (uint32_t)__bfloat16_as_ushort(__hneg(hi)) | ((uint32_t)__bfloat16_as_ushort(__hneg(mid)) << 16);
+    w1 = (uint32_t)__bfloat16_as_ushort(__hneg(lo));
+  }
+  // two chunks of the row carry the 16 columns of a k-step
+  *reinterpret_cast<uint4*>(xt + swz(r, 0)) = kv0;
+  *reinterpret_cast<uint4*>(xt + swz(r, 1)) = make_uint4(0, 0, 0, 0);
+  *reinterpret_cast<uint4*>(xt + swz(r, 2)) = make_uint4(w0, w1, 0, 0);
+  *reinterpret_cast<uint4*>(xt + swz(r, 3)) = make_uint4(0, 0, 0, 0);
+  // Q rows (through the permutation if given)
+  int src = -1;
+  if (rr < rows_valid) {
+    src = q_row0 + rr;
+    if (perm != nullptr) src = static_cast<int>(perm[src]);
+  }
+#pragma unroll
+  for (int i = 0; i < 32 / kRowsPerInstr; ++i) {
+    const int rl = i * kRowsPerInstr + sub;
+    const int id = __shfl_sync(0xffffffffu, src, rl);
+    const uint32_t dst = s_base + L::kQ + swz<L::kQRows>(row0 + rl, cch);
+    if (c_in_tile) {
+      if (id >= 0 && c_live) cp_async16(dst, qb + cch * 16 + (size_t)id * q_row);
+      else cp_async16_zfill(dst, qb, 0);
+    }
+  }
+}
+
 template <int D, bool kFp16, int G>
 __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMassParams p, const __grid_constant__ KeyTileMap kmap, int splits) {
   // key tiles are 128 consecutive rows: with a valid tensor map one elected thread loads them by TMA
@@ -136,69 +198,15 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // one lane per 16-byte chunk of a row; the padded layouts give every lane one of 32 chunk positions, of which
-  // D / 8 exist in the tile (the others idle) and p.D / 8 hold data (the rest is zero-filled)
-  constexpr int kChunks = kWide ? 32 : D / 8;
-  constexpr int kRowsPerInstr = 32 / kChunks;
-  const int sub = lane / kChunks, cch = lane % kChunks;
-  const bool c_in_tile = !kWide || cch < D / 8;
-  const bool c_live = !kWide || cch < d_chunks;
-  // ---- constant extra K block, extra Q block, Q rows: a block of 32 rows for each of the first exponentiating warps, which would
-  // wait for scores anyway; the producers start on the keys at once.  (By the producers, before their first key tile: 9.3 us
-  // instead of 6.6 for one group against one tile at D = 96 to 192.)
+  // The query operand: a block of 32 rows for each of the first exponentiating warps, which would wait for scores anyway; the
+  // producers start on the keys at once.  (By the producers, before their first key tile: 9.3 us instead of 6.6 for one group
+  // against one tile at D = 96 to 192.)
   if (warp < L::kQRows / 32) {
-    const int row0 = warp * 32;
-    // K extra: every row (1, 1, 1, 0, ...); Q extra: (-hi, -mid, -lo, 0, ...) of lse / scale
-    const uint32_t one = kFp16 ? 0x3C00u : 0x3F80u;
-    uint8_t* xt = smem + L::kX;
-    const int r = row0 + lane;
-    uint4 kv0 = make_uint4(one | (one << 16), one, 0, 0);
-    float x = 3.0e38f;                                 // padding rows: exp(-huge) = 0
-    if (kFp16) x = 60000.f;
-    const int m = m0 + (r >> 7), rr = r & 127, q_row0 = m * p.group_rows;
-    const int rows_valid = rows_of(m);
-    if (rr < rows_valid) x = p.lse[(size_t)bh * p.Lq + q_row0 + rr] * p.inv_scale;
-    uint32_t w0, w1;
-    if (kFp16) {
-      const __half hi = __float2half_rn(x);
-      const float r1 = x - __half2float(hi);
-      const __half mid = __float2half_rn(r1);
-      const __half lo = __float2half_rn(r1 - __half2float(mid));
-      w0 = (uint32_t)__half_as_ushort(__hneg(hi)) | ((uint32_t)__half_as_ushort(__hneg(mid)) << 16);
-      w1 = (uint32_t)__half_as_ushort(__hneg(lo));
-    } else {
-      const __nv_bfloat16 hi = __float2bfloat16_rn(x);
-      const float r1 = x - __bfloat162float(hi);
-      const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
-      const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-      w0 = (uint32_t)__bfloat16_as_ushort(__hneg(hi)) | ((uint32_t)__bfloat16_as_ushort(__hneg(mid)) << 16);
-      w1 = (uint32_t)__bfloat16_as_ushort(__hneg(lo));
-    }
-    // two chunks of the row carry the 16 columns of a k-step
-    *reinterpret_cast<uint4*>(xt + swz(r, 0)) = kv0;
-    *reinterpret_cast<uint4*>(xt + swz(r, 1)) = make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(xt + swz(r, 2)) = make_uint4(w0, w1, 0, 0);
-    *reinterpret_cast<uint4*>(xt + swz(r, 3)) = make_uint4(0, 0, 0, 0);
-    // Q rows (through the permutation if given)
-    int src = -1;
-    if (rr < rows_valid) {
-      src = q_row0 + rr;
-      if (p.perm != nullptr) src = static_cast<int>(p.perm[(size_t)bh * p.Lq + src]);
-    }
-    const uint8_t* qb = reinterpret_cast<const uint8_t*>(p.q) + 2 * ((size_t)b * p.q_stride[0] + (size_t)h * p.q_stride[2]) + cch * 16;
-    const size_t q_row = 2 * (size_t)p.q_stride[1];
-#pragma unroll
-    for (int i = 0; i < 32 / kRowsPerInstr; ++i) {
-      const int rl = i * kRowsPerInstr + sub;
-      const int id = __shfl_sync(0xffffffffu, src, rl);
-      const uint32_t dst = s_base + L::kQ + swz<L::kQRows>(row0 + rl, cch);
-      if (c_in_tile) {
-        if (id >= 0 && c_live) cp_async16(dst, qb + (size_t)id * q_row);
-        else cp_async16_zfill(dst, p.q, 0);
-      }
-    }
+    prepare_queries<D, kFp16, G>(smem, p.lse + (size_t)bh * p.Lq, p.perm == nullptr ? nullptr : p.perm + (size_t)bh * p.Lq,
+                                 reinterpret_cast<const uint8_t*>(p.q) + 2 * ((size_t)b * p.q_stride[0] + (size_t)h * p.q_stride[2]),
+                                 2 * (size_t)p.q_stride[1], m0, p.M, p.group_rows, p.Lq, p.inv_scale, d_chunks, warp * 32);
     fence_proxy_async_smem();
-    mbar_arrive(bar(BAR_Q_FULL));                      // release: the plain stores above
+    mbar_arrive(bar(BAR_Q_FULL));                        // release: the plain stores above
     cp_async_arrive_noinc(bar(BAR_Q_FULL));
   }
 
@@ -327,6 +335,13 @@ __global__ void __launch_bounds__(kThreads, 1) group_mass_kernel(const GroupMass
   } else {
     // ===================================================================== producers
     const int pw = warp - kProducerWarp0;
+    // one lane per 16-byte chunk of a row; the padded layouts give every lane one of 32 chunk positions, of which
+    // D / 8 exist in the tile (the others idle) and p.D / 8 hold data (the rest is zero-filled)
+    constexpr int kChunks = kWide ? 32 : D / 8;
+    constexpr int kRowsPerInstr = 32 / kChunks;
+    const int sub = lane / kChunks, cch = lane % kChunks;
+    const bool c_in_tile = !kWide || cch < D / 8;
+    const bool c_live = !kWide || cch < d_chunks;
     // ---- key tiles: contiguous rows t*128 .. t*128+127 of this head
     int n_tiles_cp = n_tiles;       // tiles copied with cp.async (none when TMA is used)
     const uint8_t* kb = reinterpret_cast<const uint8_t*>(p.k) + 2 * ((size_t)b * p.k_stride[0] + (size_t)h * p.k_stride[2]) + cch * 16;
